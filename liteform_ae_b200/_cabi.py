@@ -129,6 +129,48 @@ def load() -> C.CDLL:
     return _lib
 
 
+_torch_mod = None
+
+
+def cuda_torch():
+    """The torch module, once a CUDA device has been seen.  The query costs several microseconds, which
+    a product of a small matrix would pay on every call, so a positive answer is kept."""
+    global _torch_mod
+    if _torch_mod is None:
+        import torch
+        if not torch.cuda.is_available():
+            raise RuntimeError("liteform_ae_b200 needs a CUDA device (there is no CPU path)")
+        torch.cuda.init()
+        _torch_mod = torch
+    return _torch_mod
+
+
+class on_device:
+    """``with torch.cuda.device(i)`` for an index that almost always is the current device already:
+    then nothing is switched and nothing has to be switched back."""
+    __slots__ = ("_index", "_guard")
+
+    def __init__(self, index: int):
+        self._index = index
+
+    def __enter__(self):
+        torch = _torch_mod
+        if torch._C._cuda_getDevice() == self._index:
+            self._guard = None
+        else:
+            self._guard = torch.cuda.device(self._index)
+            self._guard.__enter__()
+
+    def __exit__(self, *exc):
+        if self._guard is not None:
+            self._guard.__exit__(*exc)
+
+
+def stream_of(index: int) -> int:
+    """Address of torch's current stream on device ``index``."""
+    return _torch_mod._C._cuda_getCurrentRawStream(index)
+
+
 def check(status: int) -> None:
     if status != LF_OK:
         msg = load().lf_last_error()

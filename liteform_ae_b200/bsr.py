@@ -15,15 +15,8 @@ from typing import Optional, Tuple
 import numpy as np
 
 from . import _cabi
-from ._cabi import check, t_ptr
+from ._cabi import check, cuda_torch as _torch, on_device, stream_of, t_ptr
 from .timing import profile_ms
-
-
-def _torch():
-    import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("liteform_ae_b200 needs a CUDA device (there is no CPU path)")
-    return torch
 
 
 @dataclass
@@ -133,15 +126,20 @@ def spmm_bsr8(a: DeviceBsr8, B, out=None, block_row_range=None):
     assert B.is_cuda and B.dim() == 2 and B.stride(1) == 1 and B.shape[0] == a.shape[1]
     assert B.dtype == a.blocks.dtype, "B and the blocks must have the same dtype"
     r0, r1 = (0, a.shape[0] // 8) if block_row_range is None else block_row_range
-    N = int(B.shape[1])
+    N = B.shape[1]
     if out is None:
         out = torch.empty(((r1 - r0) * 8, N), dtype=torch.float32, device=B.device)
-    assert out.dtype == torch.float32 and out.shape == ((r1 - r0) * 8, N) and out.stride(1) == 1
-    fn = {torch.float32: lib.lf_spmm_bsr8_f32, torch.bfloat16: lib.lf_spmm_bsr8_bf16,
-          torch.float16: lib.lf_spmm_bsr8_f16}[a.blocks.dtype]
-    with torch.cuda.device(B.device):
+    else:
+        assert out.dtype == torch.float32 and out.shape == ((r1 - r0) * 8, N) and out.stride(1) == 1
+    dtype = B.dtype
+    if dtype is torch.float32:
+        fn = lib.lf_spmm_bsr8_f32
+    else:
+        fn = {torch.bfloat16: lib.lf_spmm_bsr8_bf16, torch.float16: lib.lf_spmm_bsr8_f16}[dtype]
+    dev = B.get_device()
+    with on_device(dev):
         check(fn(t_ptr(a.indptr), t_ptr(a.indices), t_ptr(a.blocks), r0, r1, B.data_ptr(), B.stride(0),
-                 out.data_ptr(), out.stride(0), N, torch.cuda.current_stream().cuda_stream))
+                 out.data_ptr(), out.stride(0), N, stream_of(dev)))
     return out
 
 

@@ -739,12 +739,6 @@ int check_common(const void* indptr, const void* indices, const void* blocks, in
   return LF_OK;
 }
 
-template <typename K>
-int set_smem(K kernel, int bytes) {
-  LF_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  return LF_OK;
-}
-
 }  // namespace
 
 // 0 = automatic, 1 = per-lane cp.async, 2 = tiled bulk copies, 3 = one bulk copy per B row
@@ -829,8 +823,8 @@ int lf_spmm_bsr8_f32(const int64_t* indptr, const int32_t* indices, const float*
   if (N <= 32 && !g_bsr_feat_units) {   // narrow tile: both halves of every MMA carry features
     const int ntiles = (N + 31) / 32;
     const int64_t ngrid = ceil_div64(groups * ntiles, kWarps);
-    auto k = bsr8_spmm_f32_narrow_kernel<6, 3>;
-    if (int s = set_smem(k, F32NarrowCfg<6>::kSmem)) return s;
+    constexpr auto k = bsr8_spmm_f32_narrow_kernel<6, 3>;
+    LF_CUDA_CHECK(allow_smem<k>(F32NarrowCfg<6>::kSmem));
     k<<<(unsigned)ngrid, kThreadsBsr, F32NarrowCfg<6>::kSmem, st>>>(indptr, indices, blocks, block_row_begin,
                                                                     block_row_end, B, (int)ldb, C, ldc, N, ntiles, rpw);
     LF_CUDA_CHECK(cudaGetLastError());
@@ -848,9 +842,9 @@ int lf_spmm_bsr8_f32(const int64_t* indptr, const int32_t* indices, const float*
   LF_REQUIRE(wgrid < (1ll << 31), "too many thread blocks");
 #define LF_BSR(T_, D_, M_)                                                                                   \
   do {                                                                                                       \
-    auto k = bsr8_spmm_f32_kernel<T_, D_, M_>;                                                               \
+    constexpr auto k = bsr8_spmm_f32_kernel<T_, D_, M_>;                                                               \
     const int smem = W * D_ * F32Cfg<T_, D_>::kStage;                                                        \
-    if (int s = set_smem(k, smem)) return s;                                                                 \
+    LF_CUDA_CHECK(allow_smem<k>(smem));                                                                 \
     k<<<(unsigned)wgrid, W * 32, smem, st>>>(indptr, indices, blocks, block_row_begin, block_row_end, B,    \
                                              (int)ldb, C, ldc, N, tiles, rpw, tile_major);                   \
   } while (0)
@@ -880,13 +874,13 @@ static int launch_16bit(bool bf16, const int64_t* indptr, const int32_t* indices
     const int ntiles = (N + 31) / 32;
     const int64_t ngrid = ceil_div64(ceil_div64(r1 - r0, rpw) * ntiles, kWarps);
     if (bf16) {
-      auto k = bsr8_spmm_16bit_narrow_kernel<true, 6, 3>;
-      if (int s = set_smem(k, H16NarrowCfg<6>::kSmem)) return s;
+      constexpr auto k = bsr8_spmm_16bit_narrow_kernel<true, 6, 3>;
+      LF_CUDA_CHECK(allow_smem<k>(H16NarrowCfg<6>::kSmem));
       k<<<(unsigned)ngrid, kThreadsBsr, H16NarrowCfg<6>::kSmem, st>>>(indptr, indices, blocks, r0, r1, B, (int)ldb, C,
                                                                       ldc, N, ntiles, rpw);
     } else {
-      auto k = bsr8_spmm_16bit_narrow_kernel<false, 6, 3>;
-      if (int s = set_smem(k, H16NarrowCfg<6>::kSmem)) return s;
+      constexpr auto k = bsr8_spmm_16bit_narrow_kernel<false, 6, 3>;
+      LF_CUDA_CHECK(allow_smem<k>(H16NarrowCfg<6>::kSmem));
       k<<<(unsigned)ngrid, kThreadsBsr, H16NarrowCfg<6>::kSmem, st>>>(indptr, indices, blocks, r0, r1, B, (int)ldb, C,
                                                                       ldc, N, ntiles, rpw);
     }
@@ -896,13 +890,13 @@ static int launch_16bit(bool bf16, const int64_t* indptr, const int32_t* indices
   if (N <= 64 && !g_bsr_stages) {   // 64 features per warp
     const int64_t ngrid = ceil_div64(ceil_div64(r1 - r0, rpw), kWarps);
     if (bf16) {
-      auto k = bsr8_spmm_16bit_mid_kernel<true, 4, 3>;
-      if (int s = set_smem(k, H16MidCfg<4>::kSmem)) return s;
+      constexpr auto k = bsr8_spmm_16bit_mid_kernel<true, 4, 3>;
+      LF_CUDA_CHECK(allow_smem<k>(H16MidCfg<4>::kSmem));
       k<<<(unsigned)ngrid, kThreadsBsr, H16MidCfg<4>::kSmem, st>>>(indptr, indices, blocks, r0, r1, B, (int)ldb, C, ldc,
                                                                    N, 1, rpw);
     } else {
-      auto k = bsr8_spmm_16bit_mid_kernel<false, 4, 3>;
-      if (int s = set_smem(k, H16MidCfg<4>::kSmem)) return s;
+      constexpr auto k = bsr8_spmm_16bit_mid_kernel<false, 4, 3>;
+      LF_CUDA_CHECK(allow_smem<k>(H16MidCfg<4>::kSmem));
       k<<<(unsigned)ngrid, kThreadsBsr, H16MidCfg<4>::kSmem, st>>>(indptr, indices, blocks, r0, r1, B, (int)ldb, C, ldc,
                                                                    N, 1, rpw);
     }
@@ -925,9 +919,9 @@ static int launch_16bit(bool bf16, const int64_t* indptr, const int32_t* indices
   LF_REQUIRE(wgrid < (1ll << 31), "too many thread blocks");
 #define LF_BSR16(B_, D_, M_)                                                                                  \
   do {                                                                                                        \
-    auto k = bsr8_spmm_16bit_kernel<B_, D_, M_>;                                                              \
+    constexpr auto k = bsr8_spmm_16bit_kernel<B_, D_, M_>;                                                              \
     const int smem = W * D_ * H16Cfg<D_>::kStage;                                                             \
-    if (int s = set_smem(k, smem)) return s;                                                                  \
+    LF_CUDA_CHECK(allow_smem<k>(smem));                                                                  \
     k<<<(unsigned)wgrid, W * 32, smem, st>>>(indptr, indices, blocks, r0, r1, B, (int)ldb, C, ldc, N, tiles, rpw); \
   } while (0)
   if (bf16) { if (D == 3) LF_BSR16(true, 3, 2); else LF_BSR16(true, 4, 1); }

@@ -1242,8 +1242,8 @@ int launch_hyb_bf16(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, 
     // more than 128 bf16 features: full warps, one thread block along y per 256 features
     dim3 rgrid((unsigned)tiles, (unsigned)((N + 255) / 256));
     const size_t smem = (size_t)(kThreads / 32) * 16 * 32 * sizeof(float4);
-    auto kern = spmm_hyb_ring_kernel<16, MAXB, 1, 3, false, 8>;
-    LF_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = spmm_hyb_ring_kernel<16, MAXB, 1, 3, false, 8>;
+    LF_CUDA_CHECK(allow_smem<kern>((int)smem));
     LF_CUDA_CHECK(launch_dep_smem(kern, rgrid, kThreads, smem, st, dep, tbl, A->rows, A->cols, A->vals, B, (int)ldb, C,
                                   ldc, N, A->row_begin, dests));
     return LF_OK;
@@ -1292,8 +1292,8 @@ int launch_hyb_ring_rows(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb
   const size_t smem = (size_t)(kThreads / 32) * 16 * 32 * sizeof(float4);
 #define LF_ROWS(R_, VEC_, T_)                                                                                   \
   do {                                                                                                          \
-    auto kern = spmm_hyb_ring_rows_kernel<R_, VEC_, MAXB, 1>;                                                   \
-    LF_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));          \
+    constexpr auto kern = spmm_hyb_ring_rows_kernel<R_, VEC_, MAXB, 1>;                                                   \
+    LF_CUDA_CHECK(allow_smem<kern>((int)smem));          \
     LF_CUDA_CHECK(launch_dep_smem(kern, grid, kThreads, smem, st, dep, tbl, A->rows, A->cols, A->vals,          \
                                   (const T_*)B, (int)ldb, C, ldc, N, A->row_begin));                            \
     return LF_OK;                                                                                               \
@@ -1321,8 +1321,8 @@ int launch_hyb(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, const
     const size_t smem = (size_t)(kThreads / 32) * ring * 32 * sizeof(float4);
 #define LF_RING(D_, P_, M_, MD_)                                                                                \
   do {                                                                                                          \
-    auto kern = spmm_hyb_ring_kernel<D_, MAXB, P_, M_, MD_, 4>;                                                 \
-    LF_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));          \
+    constexpr auto kern = spmm_hyb_ring_kernel<D_, MAXB, P_, M_, MD_, 4>;                                                 \
+    LF_CUDA_CHECK(allow_smem<kern>((int)smem));          \
     LF_CUDA_CHECK(launch_dep_smem(kern, grid, kThreads, smem, st, dep, tbl, A->rows, A->cols, A->vals, B,       \
                                   (int)ldb, C, ldc, N, MD_ ? (int64_t)0 : A->row_begin, dests));                \
     return LF_OK;                                                                                               \
@@ -1710,8 +1710,8 @@ int lf_spmm_csr_f32(const int64_t* indptr, const int32_t* indices, const float* 
   if (gather_ring() > 0 && ring_applies(cfg, ldb)) {
     dim3 rgrid((unsigned)blocks, (unsigned)((N + kRingFeatures - 1) / kRingFeatures));
     const size_t smem = (size_t)(kThreads / 32) * 16 * 32 * sizeof(float4);
-    auto kern = spmm_csr_ring_kernel<16>;
-    LF_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr auto kern = spmm_csr_ring_kernel<16>;
+    LF_CUDA_CHECK(allow_smem<kern>((int)smem));
     LF_CUDA_CHECK(launch_dep_smem(kern, rgrid, kThreads, smem, st, true, indptr, indices, data, row_begin, row_end, B,
                                   (int)ldb, C, ldc, N, spg));
     return LF_OK;

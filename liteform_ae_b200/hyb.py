@@ -12,16 +12,9 @@ from typing import List, Optional, Sequence, Tuple
 import numpy as np
 
 from . import _cabi
-from ._cabi import LfHyb, check, np_ptr, t_ptr
+from ._cabi import LfHyb, check, cuda_torch as _torch, np_ptr, on_device, stream_of, t_ptr
 
 BUCKET_ALIGN = 64
-
-
-def _torch():
-    import torch
-    if not torch.cuda.is_available():
-        raise RuntimeError("liteform_ae_b200 needs a CUDA device (there is no CPU path)")
-    return torch
 
 
 def _stream_ptr(torch) -> int:
@@ -144,6 +137,25 @@ class HybFormat:
         self.row_off = np.ascontiguousarray(row_off, dtype=np.int64)
         self.slot_off = np.ascontiguousarray(slot_off, dtype=np.int64)
         self.rows, self.cols, self.vals, self.mask, self.zero_rows = rows, cols, vals, mask, zero_rows
+
+    def __setattr__(self, name, value):
+        self.__dict__[name] = value
+        self.__dict__["_c_view"] = None      # any attribute may be part of the C view kept below
+
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_c_view"}
+
+    def _c_ref(self):
+        """``byref`` of ``c_struct()``, kept until an attribute is assigned or a device array changes its
+        address: filling the structure costs more host time than a small product takes on the device."""
+        z = self.zero_rows
+        now = (self.rows.data_ptr(), self.cols.data_ptr(), self.vals.data_ptr(), -1 if z is None else z.data_ptr())
+        kept = self.__dict__.get("_c_view")
+        if kept is None or kept[0] != now:
+            s = self.c_struct()
+            kept = (now, C.byref(s), s)
+            self.__dict__["_c_view"] = kept
+        return kept[1]
 
     # -- C view ---------------------------------------------------------------------------
     def c_struct(self, host_arrays=None) -> LfHyb:
@@ -307,21 +319,22 @@ def spmm_hyb(fmt: HybFormat, B, out=None, accumulate: bool = False):
     ``C[row_begin:row_end]`` (float32, on the format's device)."""
     torch = _torch()
     lib = _cabi.load()
-    assert B.is_cuda and B.dtype in (torch.float32, torch.bfloat16) and B.dim() == 2 and B.stride(1) == 1
-    assert B.shape[0] == fmt.shape[1], "B must have one row per matrix column"
-    N = int(B.shape[1])
+    dtype = B.dtype
+    assert B.is_cuda and B.dim() == 2 and B.stride(1) == 1 and dtype in (torch.float32, torch.bfloat16)
+    K, N = B.shape
+    assert K == fmt.shape[1], "B must have one row per matrix column"
     n_rows = fmt.row_end - fmt.row_begin
     if out is None:
         if accumulate:
             raise ValueError("accumulate=True needs an output tensor")
         out = torch.empty((n_rows, N), dtype=torch.float32, device=B.device)
-    assert out.shape == (n_rows, N) and out.stride(1) == 1 and out.dtype == torch.float32
-    with torch.cuda.device(B.device):
-        s = fmt.c_struct()
-        fn = lib.lf_spmm_hyb_f32 if B.dtype == torch.float32 else lib.lf_spmm_hyb_bf16
-        check(fn(C.byref(s), B.data_ptr(), B.stride(0), out.data_ptr(), out.stride(0), N,
-                                  _cabi.LF_SPMM_ACCUMULATE if accumulate else _cabi.LF_SPMM_OVERWRITE,
-                                  _stream_ptr(torch)))
+    else:
+        assert out.shape == (n_rows, N) and out.stride(1) == 1 and out.dtype == torch.float32
+    dev = B.get_device()
+    with on_device(dev):
+        fn = lib.lf_spmm_hyb_f32 if dtype is torch.float32 else lib.lf_spmm_hyb_bf16
+        check(fn(fmt._c_ref(), B.data_ptr(), B.stride(0), out.data_ptr(), out.stride(0), N,
+                 _cabi.LF_SPMM_ACCUMULATE if accumulate else _cabi.LF_SPMM_OVERWRITE, stream_of(dev)))
     return out
 
 
@@ -339,14 +352,14 @@ def spmm_csr(csr: DeviceCsr, B, out=None, row_range=None):
     lib = _cabi.load()
     assert B.is_cuda and B.dtype == torch.float32 and B.stride(1) == 1
     r0, r1 = (0, csr.shape[0]) if row_range is None else row_range
-    N = int(B.shape[1])
+    N = B.shape[1]
     if out is None:
         out = torch.empty((r1 - r0, N), dtype=torch.float32, device=B.device)
-    with torch.cuda.device(B.device):
+    dev = B.get_device()
+    with on_device(dev):
         nnz = csr.nnz if (r0, r1) == (0, csr.shape[0]) else -1
         check(lib.lf_spmm_csr_f32(t_ptr(csr.indptr), t_ptr(csr.indices), t_ptr(csr.data), r0, r1, nnz,
-                                  B.data_ptr(), B.stride(0), out.data_ptr(), out.stride(0), N,
-                                  _stream_ptr(torch)))
+                                  B.data_ptr(), B.stride(0), out.data_ptr(), out.stride(0), N, stream_of(dev)))
     return out
 
 
