@@ -28,15 +28,36 @@
 //     or 16 lanes, several slots per step);
 //   * variants of the same code: B in bf16 (8 features per lane), and a broadcasting epilogue that
 //     stores every row into several full-size C matrices (the GPUs of a group) at once.
-#include <type_traits>
-
 #include "lf_bsr8_tma.cuh"
-#include "lf_common.cuh"
+#include "lf_spmm_gather.cuh"
 
 namespace lf {
-namespace {
 
-constexpr int kThreads = 256;
+int sm_count() {
+  static int cached[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if (!cached[dev]) {
+    int n = 0;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
+    cached[dev] = n;
+  }
+  return cached[dev];
+}
+
+constexpr int kDefaultGatherRing = 16;
+int g_gather_ring = -1;
+// Depth of the shared-memory gather ring (rows in flight per warp): 0 = gathers land in registers.
+int gather_ring() {
+  if (g_gather_ring < 0) {
+    const char* e = getenv("LF_SPMM_GATHER_RING");
+    const int v = e ? atoi(e) : kDefaultGatherRing;
+    g_gather_ring = (v == 0 || v == 16) ? v : kDefaultGatherRing;
+  }
+  return g_gather_ring;
+}
+
+namespace {
 
 struct BucketDesc {
   int64_t row_off;        // first element of this bucket in the rows arena
@@ -61,88 +82,6 @@ struct SpmmTable {
   int32_t seg_tiles;      // thread blocks per segment over all buckets (0 = bucket-major)
   BucketDesc b[MAXB];
 };
-
-// Destinations of a broadcasting launch: full-size C matrices (row 0 first), one per GPU of the
-// group, addressed through peer mappings; the shard's rows are written into every one of them.
-struct DestList {
-  float* p[LF_MAX_DESTS];
-  int32_t n;
-  int32_t pad_;
-};
-
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
-}
-
-// Programmatic dependent launch: the product kernel is launched while the launch that clears
-// rows is still running; everything up to this point (bucket look-up, first loads) overlaps with
-// it, and nothing is written to C before the clearing launch has completed and flushed.  Without
-// a programmatic dependency the instruction returns at once.
-__device__ __forceinline__ void wait_for_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void let_dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-template <int VEC> struct Chunk;
-template <> struct Chunk<4> {
-  float4 v;
-  __device__ __forceinline__ void zero() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ __forceinline__ void load(const float* p) { v = __ldg(reinterpret_cast<const float4*>(p)); }
-  __device__ __forceinline__ void store_stream(float* p) const { __stcs(reinterpret_cast<float4*>(p), v); }
-  __device__ __forceinline__ void fma(float a, const Chunk& x) {
-    v.x = fmaf(a, x.v.x, v.x); v.y = fmaf(a, x.v.y, v.y); v.z = fmaf(a, x.v.z, v.z); v.w = fmaf(a, x.v.w, v.w);
-  }
-  __device__ __forceinline__ void store(float* p) const { *reinterpret_cast<float4*>(p) = v; }
-  __device__ __forceinline__ void red(float* p) const { red_add_v4(p, v.x, v.y, v.z, v.w); }
-};
-template <> struct Chunk<1> {
-  float v;
-  __device__ __forceinline__ void zero() { v = 0.f; }
-  __device__ __forceinline__ void load(const float* p) { v = __ldg(p); }
-  __device__ __forceinline__ void store_stream(float* p) const { __stcs(p, v); }
-  __device__ __forceinline__ void fma(float a, const Chunk& x) { v = fmaf(a, x.v, v); }
-  __device__ __forceinline__ void store(float* p) const { *p = v; }
-  __device__ __forceinline__ void red(float* p) const { atomicAdd(p, v); }
-};
-
-// VEC = 8 stands for "B holds bf16": a lane gathers 8 consecutive 16-bit features with one
-// 128-bit load and accumulates them in 8 floats (fp32 accumulation, fp32 C).
-template <> struct Chunk<8> {
-  float a[8];
-  __device__ __forceinline__ void zero() {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) a[i] = 0.f;
-  }
-  __device__ __forceinline__ void store(float* p) const {
-    *reinterpret_cast<float4*>(p) = make_float4(a[0], a[1], a[2], a[3]);
-    *reinterpret_cast<float4*>(p + 4) = make_float4(a[4], a[5], a[6], a[7]);
-  }
-  __device__ __forceinline__ void store_stream(float* p) const {
-    __stcs(reinterpret_cast<float4*>(p), make_float4(a[0], a[1], a[2], a[3]));
-    __stcs(reinterpret_cast<float4*>(p + 4), make_float4(a[4], a[5], a[6], a[7]));
-  }
-  __device__ __forceinline__ void red(float* p) const {
-    red_add_v4(p, a[0], a[1], a[2], a[3]);
-    red_add_v4(p + 4, a[4], a[5], a[6], a[7]);
-  }
-};
-struct RawBf16x8 {
-  uint4 v;
-  __device__ __forceinline__ void zero() { v = make_uint4(0u, 0u, 0u, 0u); }
-  __device__ __forceinline__ void load(const uint16_t* p) { v = __ldg(reinterpret_cast<const uint4*>(p)); }
-};
-// element type of B and the register image of one gathered chunk, per VEC
-template <int VEC> struct BTraits { using elem = float; using raw = Chunk<VEC>; };
-template <> struct BTraits<8> { using elem = uint16_t; using raw = RawBf16x8; };
-
-__device__ __forceinline__ void chunk_fma(Chunk<4>& acc, float a, const Chunk<4>& x) { acc.fma(a, x); }
-__device__ __forceinline__ void chunk_fma(Chunk<1>& acc, float a, const Chunk<1>& x) { acc.fma(a, x); }
-__device__ __forceinline__ void chunk_fma(Chunk<8>& acc, float a, const RawBf16x8& x) {
-  const uint32_t w[4] = {x.v.x, x.v.y, x.v.z, x.v.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {   // a bf16 is the upper half of the float with the same value
-    acc.a[2 * i] = fmaf(a, __uint_as_float(w[i] << 16), acc.a[2 * i]);
-    acc.a[2 * i + 1] = fmaf(a, __uint_as_float(w[i] & 0xffff0000u), acc.a[2 * i + 1]);
-  }
-}
 
 // One thread group walks the slots [s0, s1) of whole ELL rows of one bucket.
 //   G lanes per group, V chunks of VEC floats per lane: one pass covers G*V*VEC features.
@@ -317,23 +256,6 @@ spmm_hyb_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int32_t* __re
 // constants and the address of a row is one multiply-add.  A warp covers 128 float32 (256 bf16)
 // features, one 16-byte chunk per lane; wider feature matrices use further thread blocks along
 // y.  Rows are added up in the same order as in the register kernel.
-__device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int PENDING>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
-
-// address of row `col` of a matrix whose rows are `pitch_bytes` apart: one 32 x 32 + 64 bit multiply-add
-__device__ __forceinline__ const void* row_of_b(const void* base, uint32_t col, uint32_t pitch_bytes) {
-  uint64_t a;
-  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(a) : "r"(col), "r"(pitch_bytes), "l"(reinterpret_cast<uint64_t>(base)));
-  return reinterpret_cast<const void*>(a);
-}
-
-constexpr int kRingFeatures = 128;   // features one warp of the ring kernel covers
-
-constexpr uint32_t kNoGather = 0xffffffffu;   // column of a slot that gathers nothing (padding, stored zero)
 
 // Everything that is the same for all lanes of a warp is computed once per slot by ONE lane while
 // a strip of 32 slots is staged ("gathers nothing" folded into the column index, "an ELL row with
@@ -764,324 +686,6 @@ zero_rows_multi_kernel(const int32_t* __restrict__ zero_rows, int64_t n, const _
   }
 }
 
-// ---------------------------------------------------------------------------------------------
-// CSR SpMM (the kernel behind bench_naive, format_algos.py:1660-1755), balanced over entries
-// instead of rows: every thread group takes `spg` consecutive stored entries, whatever rows they
-// belong to, so a 100 000-entry row is shared by hundreds of groups and short rows are packed
-// together.  A row that lies inside one group's range is written with a plain store; a row cut
-// by a range boundary is accumulated with vector atomics after csr_prepare_kernel cleared it.
-// ---------------------------------------------------------------------------------------------
-// One warp per candidate: lane 0 decides which rows (at most two) have to be cleared, the warp
-// clears them with coalesced (128-bit when VEC == 4) stores.
-template <int VEC>
-__global__ void __launch_bounds__(256)
-csr_prepare_kernel(const int64_t* __restrict__ indptr, int64_t row_begin, int64_t row_end, int64_t spg,
-                   float* __restrict__ C, int64_t ldc, int N) {
-  let_dependents_launch();
-  const int lane = threadIdx.x & 31;
-  const int64_t rows = row_end - row_begin;
-  const int64_t base = indptr[row_begin];
-  const int64_t total = indptr[row_end] - base;
-  const int64_t groups = (total + spg - 1) / spg;
-  const int64_t n = rows > groups ? rows : groups;
-  const int64_t n_warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  auto clear = [&](int64_t row) {
-    float* dst = C + row * ldc;
-    if (VEC == 4) {
-      for (int f = lane * 4; f < N; f += 128) *reinterpret_cast<float4*>(dst + f) = make_float4(0.f, 0.f, 0.f, 0.f);
-    } else {
-      for (int f = lane; f < N; f += 32) dst[f] = 0.f;
-    }
-  };
-  for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += n_warps) {
-    int64_t empty_row = -1, cut_row = -1;
-    if (lane == 0) {
-      if (i < rows && indptr[row_begin + i] == indptr[row_begin + i + 1]) empty_row = i;
-      if (i >= 1 && i < groups) {   // the row that contains the first entry of group i, if it started earlier
-        const int64_t x = base + i * spg;
-        int64_t lo = row_begin, hi = row_end;   // indptr[lo] <= x, answer in [lo, hi)
-        while (hi - lo > 1) {
-          const int64_t mid = (lo + hi) >> 1;
-          if (indptr[mid] <= x) lo = mid; else hi = mid;
-        }
-        if (indptr[lo] < x) cut_row = lo - row_begin;
-      }
-    }
-    empty_row = __shfl_sync(0xffffffffu, empty_row, 0);
-    cut_row = __shfl_sync(0xffffffffu, cut_row, 0);
-    if (empty_row >= 0) clear(empty_row);
-    if (cut_row >= 0) clear(cut_row);
-  }
-}
-
-template <int G, int V, int VEC>
-__global__ void __launch_bounds__(kThreads, 3)
-spmm_csr_kernel(const int64_t* __restrict__ indptr, const int32_t* __restrict__ indices,
-                const float* __restrict__ data, int64_t row_begin, int64_t row_end,
-                const float* __restrict__ B, int ldb, float* __restrict__ C, int64_t ldc, int N, int spg) {
-  constexpr int GPC = kThreads / G;
-  constexpr int U = V == 1 ? 8 : (V == 2 ? 4 : 2);
-  __shared__ int2 s_cv[kThreads];
-  __shared__ int64_t s_bd[kThreads];
-  const int g = threadIdx.x / G, lane = threadIdx.x % G;
-  const int shift = (threadIdx.x & 31) / G * G;
-  const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << shift);
-  const int64_t base = indptr[row_begin];
-  const int64_t total = indptr[row_end] - base;
-  const int64_t s0 = ((int64_t)blockIdx.x * GPC + g) * (int64_t)spg;
-  if (s0 >= total) return;
-  const int64_t s1 = min(s0 + spg, total);
-  int2* cv = s_cv + g * G;
-  int64_t* bd = s_bd + g * G;
-
-  // (G+1)-ary search, one probe per lane: the row that holds entry s0
-  int64_t lo = row_begin, hi = row_end;   // indptr[lo] - base <= s0, answer in [lo, hi)
-  while (hi - lo > 1) {
-    const int64_t span = hi - lo;
-    int64_t q = lo + ((int64_t)(lane + 1) * span) / (G + 1);
-    if (q <= lo) q = lo + 1;
-    const bool le = indptr[q] - base <= s0;
-    const int cnt = __popc((__ballot_sync(gmask, le) & gmask) >> shift);   // probes are monotone
-    const int64_t qlo = __shfl_sync(gmask, q, cnt > 0 ? cnt - 1 : 0, G);
-    const int64_t qhi = __shfl_sync(gmask, q, cnt < G ? cnt : G - 1, G);
-    if (cnt > 0) lo = qlo;
-    if (cnt < G) hi = qhi;
-  }
-  int64_t cur = lo;
-  const int64_t first_row = cur;
-  const bool head_open = indptr[cur] - base < s0;
-
-  // boundaries of the next G rows, refilled when used up
-  int kb = 0;
-  auto refill = [&]() {
-    __syncwarp(gmask);
-    const int64_t r = cur + 1 + lane;
-    bd[lane] = indptr[r < row_end ? r : row_end] - base;
-    __syncwarp(gmask);
-    kb = 0;
-  };
-  refill();
-  int64_t nb = bd[0];   // first entry of the next row
-
-  const int f0 = blockIdx.y * (G * V * VEC) + lane * VEC;
-  bool active[V];
-  Chunk<VEC> acc[V];
-#pragma unroll
-  for (int v = 0; v < V; ++v) { active[v] = f0 + v * G * VEC < N; acc[v].zero(); }
-
-  auto flush = [&](int64_t row, bool open) {
-    float* dst = C + (row - row_begin) * ldc + f0;
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-      if (active[v]) {
-        if (open) acc[v].red(dst + v * G * VEC); else acc[v].store_stream(dst + v * G * VEC);
-      }
-      acc[v].zero();
-    }
-  };
-
-  const float* __restrict__ Bf = B + f0;
-  wait_for_prior_grid();   // csr_prepare_kernel has cleared the rows that receive atomics
-  for (int64_t s = s0; s < s1; s += G) {
-    const int64_t idx = s + lane;
-    const bool in = idx < s1;
-    const int my_col = in ? __ldcs(indices + base + idx) : 0;
-    const float my_val = in ? (data ? __ldcs(data + base + idx) : 1.f) : 0.f;
-    __syncwarp(gmask);
-    cv[lane] = make_int2(my_col, __float_as_int(my_val));
-    __syncwarp(gmask);
-    const int nstrip = (int)min((int64_t)G, s1 - s);
-    for (int t = 0; t < nstrip; t += U) {
-      float val[U];
-      Chunk<VEC> b[U][V];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int2 p = cv[t + u];
-        val[u] = __int_as_float(p.y);
-        const float* src = Bf + (int64_t)p.x * ldb;
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-          if (val[u] != 0.f && active[v]) b[u][v].load(src + v * G * VEC); else b[u][v].zero();
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int64_t pos = s + t + u;
-        if (pos < s1) {
-          while (pos == nb) {   // the current row ended here (and empty rows may follow)
-            flush(cur, cur == first_row && head_open);
-            ++cur;
-            if (++kb == G) refill();
-            nb = bd[kb];
-          }
-#pragma unroll
-          for (int v = 0; v < V; ++v) acc[v].fma(val[u], b[u][v]);
-        }
-      }
-    }
-  }
-  flush(cur, (cur == first_row && head_open) || s1 < nb);
-}
-
-// The CSR product with the gathers staged through the same per-lane shared-memory ring as
-// spmm_hyb_ring_kernel: a warp takes `spg` consecutive entries and 128 features, copies rows of B
-// 16 entries ahead of the one it is adding up, and follows the row boundaries exactly like the
-// register kernel above (same order of additions, same flush rules).
-template <int D>
-__global__ void __launch_bounds__(kThreads, 3)
-spmm_csr_ring_kernel(const int64_t* __restrict__ indptr, const int32_t* __restrict__ indices,
-                     const float* __restrict__ data, int64_t row_begin, int64_t row_end,
-                     const float* __restrict__ B, int ldb, float* __restrict__ C, int64_t ldc, int N, int spg) {
-  constexpr int GPC = kThreads / 32, U = 8;
-  static_assert(D == 2 * U, "two commit groups of eight rows");
-  extern __shared__ __align__(16) unsigned char ring_bytes[];
-  __shared__ __align__(16) uint32_t s_off[GPC * 64];
-  __shared__ __align__(16) float s_val[GPC * 64];
-  __shared__ int64_t s_bd[kThreads];
-  const int g = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t base = indptr[row_begin];
-  const int64_t total = indptr[row_end] - base;
-  const int64_t s0 = ((int64_t)blockIdx.x * GPC + g) * (int64_t)spg;
-  if (s0 >= total) return;
-  const int64_t s1 = min(s0 + spg, total);
-  uint32_t* so = s_off + g * 64;
-  float* sv = s_val + g * 64;
-  int64_t* bd = s_bd + g * 32;
-
-  // 33-ary search, one probe per lane: the row that holds entry s0
-  int64_t lo = row_begin, hi = row_end;   // indptr[lo] - base <= s0, answer in [lo, hi)
-  while (hi - lo > 1) {
-    const int64_t span = hi - lo;
-    int64_t q = lo + ((int64_t)(lane + 1) * span) / 33;
-    if (q <= lo) q = lo + 1;
-    const bool le = indptr[q] - base <= s0;
-    const int cnt = __popc(__ballot_sync(0xffffffffu, le));   // probes are monotone
-    const int64_t qlo = __shfl_sync(0xffffffffu, q, cnt > 0 ? cnt - 1 : 0);
-    const int64_t qhi = __shfl_sync(0xffffffffu, q, cnt < 32 ? cnt : 31);
-    if (cnt > 0) lo = qlo;
-    if (cnt < 32) hi = qhi;
-  }
-  int64_t cur = lo;
-  const int64_t first_row = cur;
-  const bool head_open = indptr[cur] - base < s0;
-
-  int kb = 0;   // boundaries of the next 32 rows, refilled when used up
-  auto refill = [&]() {
-    __syncwarp();
-    const int64_t r = cur + 1 + lane;
-    bd[lane] = indptr[r < row_end ? r : row_end] - base;
-    __syncwarp();
-    kb = 0;
-  };
-  refill();
-  int64_t nb = bd[0];   // first entry of the next row
-
-  const int f0 = blockIdx.y * kRingFeatures + lane * 4;
-  const bool active = f0 < N;
-  Chunk<4> acc;
-  acc.zero();
-  auto flush = [&](int64_t row, bool open) {
-    float* dst = C + (row - row_begin) * ldc + f0;
-    if (active) {
-      if (open) acc.red(dst); else acc.store_stream(dst);
-    }
-    acc.zero();
-  };
-
-  const float* __restrict__ Bf = B + f0;
-  const int n = (int)(s1 - s0);
-  const int nstrips = (n + 31) >> 5;
-  int pc = 0;
-  float pv = 0.f;
-  auto load_strip = [&](int k) {
-    const int64_t idx = s0 + (int64_t)k * 32 + lane;
-    const bool in = idx < s1;
-    pc = in ? __ldcs(indices + base + idx) : 0;
-    pv = in ? (data ? __ldcs(data + base + idx) : 1.f) : 0.f;
-  };
-  auto store_strip = [&](int k) {
-    const int h = (k & 1) * 32 + lane;
-    so[h] = pv != 0.f ? (uint32_t)pc : kNoGather;
-    sv[h] = pv;
-  };
-  load_strip(0);
-  store_strip(0);
-  __syncwarp();
-  if (nstrips > 1) load_strip(1);
-
-  const float4* ring_lane = reinterpret_cast<const float4*>(ring_bytes) + (size_t)g * D * 32 + lane;
-  const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring_lane);
-  const uint32_t pitch = (uint32_t)ldb * 4u;
-  const uint4* so4 = reinterpret_cast<const uint4*>(so);
-  const float4* sv4 = reinterpret_cast<const float4*>(sv);
-  auto issue_batch = [&](int j0, auto slot_tag) {
-    constexpr int SLOT = decltype(slot_tag)::value;
-    if (j0 < nstrips * 32) {
-      if ((j0 & 31) == 0 && j0 > 0) {
-        const int k = j0 >> 5;
-        __syncwarp();
-        store_strip(k);
-        __syncwarp();
-        if (k + 1 < nstrips) load_strip(k + 1);
-      }
-      const uint4 oa = so4[(j0 & 63) >> 2], ob = so4[((j0 & 63) >> 2) + 1];
-      const uint32_t o[U] = {oa.x, oa.y, oa.z, oa.w, ob.x, ob.y, ob.z, ob.w};
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (o[u] != kNoGather && active) cp_async_16(ring_s + (uint32_t)(SLOT + u) * 512u, row_of_b(Bf, o[u], pitch));
-    }
-    cp_async_commit();
-  };
-  auto for_each_batch = [&](auto&& body) {
-    body(std::integral_constant<int, 0>{});
-    body(std::integral_constant<int, U>{});
-  };
-
-  for_each_batch([&](auto slot_tag) { issue_batch(decltype(slot_tag)::value, slot_tag); });
-  wait_for_prior_grid();   // csr_prepare_kernel has cleared the rows that receive atomics
-  for (int jc0 = 0; jc0 < n; jc0 += D) {
-    for_each_batch([&](auto slot_tag) {
-      constexpr int SLOT = decltype(slot_tag)::value;
-      const int jc = jc0 + SLOT;
-      if (jc >= n) return;
-      const float4 va = sv4[(jc & 63) >> 2], vb = sv4[((jc & 63) >> 2) + 1];
-      const float val[U] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
-      const int64_t pos0 = s0 + jc;
-      cp_async_wait<D / U - 1>();
-      if (nb >= pos0 + U) {   // no row ends inside these eight entries
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (val[u] != 0.f && active) {
-            Chunk<4> x;
-            x.v = ring_lane[(SLOT + u) * 32];
-            acc.fma(val[u], x);
-          }
-        }
-      } else {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int64_t pos = pos0 + u;
-          if (pos < s1) {
-            while (pos == nb) {   // the current row ended here (and empty rows may follow)
-              flush(cur, cur == first_row && head_open);
-              ++cur;
-              if (++kb == 32) refill();
-              nb = bd[kb];
-            }
-            if (val[u] != 0.f && active) {
-              Chunk<4> x;
-              x.v = ring_lane[(SLOT + u) * 32];
-              acc.fma(val[u], x);
-            }
-          }
-        }
-      }
-      issue_batch(jc + D, slot_tag);
-    });
-  }
-  flush(cur, (cur == first_row && head_open) || s1 < nb);
-}
-
 // Ragged all-gather of C over peer mappings: the rows of this rank's block are read once and
 // stored into the same rows of every destination (plain 128-bit peer stores over NVLink).
 template <int VEC>
@@ -1104,51 +708,6 @@ allgather_rows_kernel(const float* __restrict__ src, int64_t ld_src, int64_t row
   }
 }
 
-struct FeatCfg { int G, V, VEC, pass; };
-
-// Kernel launch with, optionally, a programmatic dependency on the previous kernel of the stream
-// (the row-clearing launch): the product kernel may start before that kernel has finished and
-// orders itself with griddepcontrol.wait.
-template <typename... Params, typename... Args>
-cudaError_t launch_dep_smem(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st,
-                            bool dependent, Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = dependent ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
-}
-template <typename... Params, typename... Args>
-cudaError_t launch_dep(void (*kernel)(Params...), dim3 grid, int threads, cudaStream_t st, bool dependent, Args... args) {
-  return launch_dep_smem(kernel, grid, threads, 0, st, dependent, args...);
-}
-
-FeatCfg pick_cfg(const void* B, int64_t ldb, const void* C, int64_t ldc, int N) {
-  const bool vec = (N % 4 == 0) && (ldb % 4 == 0) && (ldc % 4 == 0) && ((uintptr_t)B % 16 == 0) &&
-                   ((uintptr_t)C % 16 == 0);
-  FeatCfg c;
-  if (vec) {
-    c.VEC = 4;
-    if (N <= 32) { c.G = 8; c.V = 1; }
-    else if (N <= 64) { c.G = 16; c.V = 1; }
-    else if (N <= 128) { c.G = 32; c.V = 1; }
-    else if (N <= 256) { c.G = 32; c.V = 2; }
-    else { c.G = 32; c.V = 4; }
-  } else {
-    c.VEC = 1;
-    c.G = 32;
-    c.V = N <= 32 ? 1 : (N <= 64 ? 2 : 4);
-  }
-  c.pass = c.G * c.V * c.VEC;
-  return c;
-}
-
 // bf16 B: 8 features per lane and chunk; needs N, ldb multiples of 8 and 16-byte aligned bases
 FeatCfg pick_cfg_bf16(int N) {
   FeatCfg c;
@@ -1162,7 +721,6 @@ FeatCfg pick_cfg_bf16(int N) {
 }
 
 // Process-wide tuning knobs (lf_set_option); the environment gives the initial values.
-constexpr int kDefaultGatherRing = 16;
 // stored slots from which rows of B narrower than a warp take the two-launch ring path (LF_OPT_SPMM_RING_MIN_SLOTS)
 int g_ring_rows_min_slots = 1 << 20;
 int g_slots_per_group = 0;
@@ -1179,18 +737,6 @@ int slots_per_group() {
     if (!g_slots_per_group && v >= 8 && v <= (1 << 20)) g_slots_per_group = v;
   }
   return g_slots_per_group;
-}
-
-int sm_count() {
-  static int cached[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-  if (!cached[dev]) {
-    int n = 0;
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
-    cached[dev] = n;
-  }
-  return cached[dev];
 }
 
 int g_tile_segments = -1;   // 0 = bucket-major order, S > 0 = interleaved over S segments
@@ -1211,17 +757,6 @@ int min_blocks() {
     g_min_blocks = (v >= 2 && v <= 4) ? v : 3;
   }
   return g_min_blocks;
-}
-
-// Depth of the shared-memory gather ring (rows in flight per warp): 0 = gathers land in registers.
-int g_gather_ring = -1;
-int gather_ring() {
-  if (g_gather_ring < 0) {
-    const char* e = getenv("LF_SPMM_GATHER_RING");
-    const int v = e ? atoi(e) : kDefaultGatherRing;
-    g_gather_ring = (v == 0 || v == 16) ? v : kDefaultGatherRing;
-  }
-  return g_gather_ring;
 }
 
 int cache_policy() {
@@ -1302,10 +837,6 @@ int launch_hyb_ring_rows(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb
   else      { if (lanes_per_row == 16) LF_ROWS(2, 4, float); else LF_ROWS(4, 4, float); }
 #undef LF_ROWS
 }
-
-// The ring kernels exist for 128-bit gathers over full warps; they multiply the column by a 32-bit
-// row pitch in bytes.
-bool ring_applies(const FeatCfg& cfg, int64_t ldb) { return cfg.VEC == 4 && cfg.G == 32 && ldb < (1ll << 30); }
 
 template <int MAXB>
 int launch_hyb(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, const void* Bv, int64_t ldb,
@@ -1672,66 +1203,6 @@ int lf_spmm_hyb_f32_host(const lf_hyb* A, const float* B, float* C, int32_t N, i
     return s;
   if (c_bytes) LF_CUDA_CHECK(cudaMemcpyAsync(C, ws + off[5], c_bytes, cudaMemcpyDeviceToHost, st));
   if (!(flags & LF_SPMM_NO_SYNC)) LF_CUDA_CHECK(cudaStreamSynchronize(st));
-  return LF_OK;
-}
-
-int lf_spmm_csr_f32(const int64_t* indptr, const int32_t* indices, const float* data, int64_t row_begin,
-                    int64_t row_end, int64_t nnz, const float* B, int64_t ldb, float* C, int64_t ldc, int32_t N,
-                    void* stream) {
-  LF_REQUIRE(N >= 1 && ldb >= N && ldc >= N && ldb < (1ll << 31), "bad arguments");
-  LF_REQUIRE(0 <= row_begin && row_begin <= row_end, "bad row range");
-  if (row_begin == row_end) return LF_OK;
-  LF_REQUIRE(indptr && B && C, "null pointer argument");
-  cudaStream_t st = (cudaStream_t)stream;
-  if (nnz < 0) {   // the launch shape depends on the number of entries: read it back
-    int64_t ends[2] = {0, 0};
-    LF_CUDA_CHECK(cudaMemcpyAsync(&ends[0], indptr + row_begin, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    LF_CUDA_CHECK(cudaMemcpyAsync(&ends[1], indptr + row_end, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    LF_CUDA_CHECK(cudaStreamSynchronize(st));
-    nnz = ends[1] - ends[0];
-  }
-  LF_REQUIRE(nnz == 0 || indices, "indices missing");
-  const FeatCfg cfg = pick_cfg(B, ldb, C, ldc, N);
-  const int gpc = kThreads / cfg.G;
-  int spg = 256;   // entries per group; smaller for small matrices so that the grid has several waves
-  while (spg > 32 && ceil_div64(nnz, (int64_t)spg * gpc) < (int64_t)sm_count() * 3 * 8) spg >>= 1;
-  {
-    const int64_t rows = row_end - row_begin, groups = ceil_div64(nnz, spg);
-    const int64_t n = rows > groups ? rows : groups;
-    const int64_t want = ceil_div64(n, 256 / 32);
-    const unsigned pgrid = (unsigned)(want > 148 * 32 ? 148 * 32 : want);
-    if (cfg.VEC == 4) csr_prepare_kernel<4><<<pgrid, 256, 0, st>>>(indptr, row_begin, row_end, spg, C, ldc, N);
-    else csr_prepare_kernel<1><<<pgrid, 256, 0, st>>>(indptr, row_begin, row_end, spg, C, ldc, N);
-    LF_CUDA_CHECK(cudaGetLastError());
-  }
-  if (nnz == 0) return LF_OK;
-  const int64_t blocks = ceil_div64(nnz, (int64_t)spg * gpc);
-  LF_REQUIRE(blocks < (1ll << 31), "too many thread blocks");
-  if (gather_ring() > 0 && ring_applies(cfg, ldb)) {
-    dim3 rgrid((unsigned)blocks, (unsigned)((N + kRingFeatures - 1) / kRingFeatures));
-    const size_t smem = (size_t)(kThreads / 32) * 16 * 32 * sizeof(float4);
-    constexpr auto kern = spmm_csr_ring_kernel<16>;
-    LF_CUDA_CHECK(allow_smem<kern>((int)smem));
-    LF_CUDA_CHECK(launch_dep_smem(kern, rgrid, kThreads, smem, st, true, indptr, indices, data, row_begin, row_end, B,
-                                  (int)ldb, C, ldc, N, spg));
-    return LF_OK;
-  }
-  dim3 grid((unsigned)blocks, (unsigned)((N + cfg.pass - 1) / cfg.pass));
-#define LF_LAUNCH(G_, V_, VEC_)                                                                              \
-  LF_CUDA_CHECK(launch_dep(spmm_csr_kernel<G_, V_, VEC_>, grid, kThreads, st, true, indptr, indices, data, row_begin, \
-                           row_end, B, (int)ldb, C, ldc, N, spg))
-  if (cfg.VEC == 4) {
-    if (cfg.G == 8) LF_LAUNCH(8, 1, 4);
-    else if (cfg.G == 16) LF_LAUNCH(16, 1, 4);
-    else if (cfg.V == 1) LF_LAUNCH(32, 1, 4);
-    else if (cfg.V == 2) LF_LAUNCH(32, 2, 4);
-    else LF_LAUNCH(32, 4, 4);
-  } else {
-    if (cfg.V == 1) LF_LAUNCH(32, 1, 1);
-    else if (cfg.V == 2) LF_LAUNCH(32, 2, 1);
-    else LF_LAUNCH(32, 4, 1);
-  }
-#undef LF_LAUNCH
   return LF_OK;
 }
 
