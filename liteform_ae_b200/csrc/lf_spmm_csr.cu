@@ -153,25 +153,26 @@ spmm_csr_kernel(const int64_t* __restrict__ indptr, const int32_t* __restrict__ 
 
 // The CSR product with the gathers staged through the group ring (lf_spmm_group.cuh): a group takes
 // spg consecutive entries, adds them up in the order of the register kernel above and flushes by the
-// same rules.  2^19 power-law rows, 7.1 M entries, 32 features: 221 us (register kernel) -> 144 us.
-template <int G, bool ODD>
-__global__ void __launch_bounds__(kThreads, 3)
+// same rules.  2^18 power-law rows, 3.7 M entries, register kernel / ring: 16 features 152 / 39 us, 64
+// features 213 / 80 us, 128 features (one row per warp and step / two) 147 / 137 us.
+template <int G, int CH, bool SH>
+__global__ void __launch_bounds__(kThreads, CH == 1 ? 4 : 3)
 spmm_csr_ring_kernel(const int64_t* __restrict__ indptr, const int32_t* __restrict__ indices,
                      const float* __restrict__ data, int64_t row_begin, int64_t row_end,
                      const float* __restrict__ B, int ldb, float* __restrict__ C, int64_t ldc, int N, int spg) {
   extern __shared__ __align__(16) unsigned char group_bytes[];
-  constexpr int R = 32 / G, kFeatures = ODD ? kGroupOddFeatures<G> : 4 * G;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int R = 32 / G, kFeatures = kGroupFeatures<G, CH, 4, SH>;
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane / G, gl = lane % G;
   const int64_t base = indptr[row_begin];
   const int64_t total = indptr[row_end] - base;
   const int64_t first = ((int64_t)blockIdx.x * (kThreads / 32) + w) * R;   // the warp's first group
   if (first * spg >= total) return;
-  const int64_t s0 = min((first + lane / G) * spg, total), s1 = min(s0 + spg, total);
+  const int64_t s0 = min((first + g) * spg, total), s1 = min(s0 + spg, total);
   CsrRowIds<G> ids;
-  ids.init(indptr + row_begin, row_end - row_begin, base, s0, s1, lane);
+  ids.init(indptr + row_begin, (int)(row_end - row_begin), base, s0, s1, g, gl);
   const int f0 = blockIdx.y * kFeatures;
-  walk_group_ring<G, 4, ODD, 1>(ids, indices + base + s0, data ? data + base + s0 : nullptr, B + f0, ldb, C + f0, ldc,
-                                min(N - f0, kFeatures), lane, group_bytes + w * GroupSmem<G, ODD>::kBytes);
+  walk_group_ring<G, CH, 4, SH, 1>(ids, false, indices + base + s0, data ? data + base + s0 : nullptr, B + f0, ldb, C + f0, ldc,
+                                   min(N - f0, kFeatures), g, gl, group_bytes + w * GroupSmem<G, CH, SH>::kBytes);
 }
 
 }  // namespace
@@ -198,12 +199,16 @@ int lf_spmm_csr_f32(const int64_t* indptr, const int32_t* indices, const float* 
   }
   LF_REQUIRE(nnz == 0 || indices, "indices missing");
   const FeatCfg cfg = pick_cfg(B, ldb, C, ldc, N);
-  // the ring form multiplies the column by a 32-bit pitch in bytes and keeps row numbers in 32 bits
-  const bool ring = gather_ring() > 0 && ldb < (1ll << 30) && row_end - row_begin < (1ll << 31) - 64;
-  const GroupCfg gcfg = pick_group(cfg.VEC == 4, N);
-  const int gpc = kThreads / (ring ? gcfg.G : cfg.G);
-  int spg = 256;   // entries per group; smaller for small matrices so that the grid has several waves
-  while (spg > 32 && ceil_div64(nnz, (int64_t)spg * gpc) < (int64_t)sm_count() * 3 * 8) spg >>= 1;
+  // the ring form multiplies row numbers by 32-bit pitches in bytes and keeps row numbers in 32 bits
+  const bool ring = gather_ring() > 0 && ldb < (1ll << 30) && ldc < (1ll << 30) && row_end - row_begin < (1ll << 31) - 64;
+  const GroupCfg group = cfg.VEC == 4 ? pick_group(N, 4) : pick_group_shifted(N);
+  const int gpc = kThreads / (ring ? group.G : cfg.G);
+  // Entries per group.  Every range boundary cuts a row (cleared before, added to twice) and costs a
+  // search, so long ranges win as soon as the grid fills the chip about twice; measured on
+  // 3.7 M entries, 16 features: 32 / 64 / 128 / 256 entries 74.8 / 68.1 / 65.4 / 63.6 us, on 1 M entries, 128
+  // features 51.3 / 45.1 / 45.3 / 51.4 us.  Below that, more blocks win until a range is one strip.
+  int spg = 256;
+  while (spg > 32 && ceil_div64(nnz, (int64_t)spg * gpc) < (int64_t)sm_count() * 3 * 2) spg >>= 1;
   const int64_t rows = row_end - row_begin;
   {
     const int spg_log = 31 - __builtin_clz((unsigned)spg);
@@ -217,23 +222,27 @@ int lf_spmm_csr_f32(const int64_t* indptr, const int32_t* indices, const float* 
   const int64_t blocks = ceil_div64(nnz, (int64_t)spg * gpc);
   LF_REQUIRE(blocks < (1ll << 31), "too many thread blocks");
   if (ring) {
-#define LF_RING(G_, ODD_)                                                                                       \
+    const dim3 rgrid((unsigned)blocks, (unsigned)group.passes);
+#define LF_RING(G_, CH_, SH_)                                                                                   \
   do {                                                                                                          \
-    constexpr auto kern = spmm_csr_ring_kernel<G_, ODD_>;                                                       \
-    constexpr int smem = kThreads / 32 * GroupSmem<G_, ODD_>::kBytes;                                           \
+    constexpr auto kern = spmm_csr_ring_kernel<G_, CH_, SH_>;                                                   \
+    constexpr int smem = kThreads / 32 * GroupSmem<G_, CH_, SH_>::kBytes;                                       \
     LF_CUDA_CHECK(allow_smem<kern>(smem));                                                                      \
-    LF_CUDA_CHECK(launch_dep_smem(kern, dim3((unsigned)blocks, (unsigned)gcfg.passes), kThreads, smem, st, true, \
-                                  indptr, indices, data, row_begin, row_end, B, (int)ldb, C, ldc, N, spg));     \
+    LF_CUDA_CHECK(launch_dep_smem(kern, rgrid, kThreads, smem, st, true, indptr, indices, data, row_begin, row_end, \
+                                  B, (int)ldb, C, ldc, N, spg));                                                \
     return LF_OK;                                                                                               \
   } while (0)
     if (cfg.VEC == 4) {
-      if (gcfg.G == 8) LF_RING(8, false);
-      else if (gcfg.G == 16) LF_RING(16, false);
-      else LF_RING(32, false);
+      if (group.G == 4) LF_RING(4, 1, false);
+      else if (group.G == 8 && group.CH == 1) LF_RING(8, 1, false);
+      else if (group.G == 8) LF_RING(8, 2, false);
+      else if (group.G == 16) LF_RING(16, 2, false);
+      else LF_RING(32, 2, false);
     } else {
-      if (gcfg.G == 8) LF_RING(8, true);
-      else if (gcfg.G == 16) LF_RING(16, true);
-      else LF_RING(32, true);
+      if (group.G == 4) LF_RING(4, 1, true);
+      else if (group.G == 8) LF_RING(8, 1, true);
+      else if (group.G == 16) LF_RING(16, 1, true);
+      else LF_RING(32, 1, true);
     }
 #undef LF_RING
   }

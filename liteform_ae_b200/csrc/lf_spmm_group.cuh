@@ -1,238 +1,297 @@
-// The gather ring for thread groups of 8, 16 or 32 lanes.
+// The gather ring for groups of lanes.
 //
-// A warp is R = 32 / G groups of G lanes; a row of B is one 16-byte chunk per lane of a group, and
-// every group walks a run of consecutive slots (entries) of its own.  Per step the warp therefore
-// multiplies R rows of B, one per group: a 128-byte row (32 float32 features) costs a quarter of the
-// instructions it would cost a whole warp.  Groups are independent -- own slots, own row
-// changes, own sum -- so a flush needs no sum over the warp and a bucket of any width (or a CSR row
-// of any length) may end at any step.  The gathers land in a ring of 16 steps in shared memory,
-// filled by cp.async; columns, values and row changes of G steps (a strip) are staged by the
-// group's lanes, one slot each, so that what is the same for all lanes is computed once.
+// A warp is R = 32 / G groups of G lanes.  A row of B is CH chunks of 16 bytes per lane of a group, and
+// every group walks a run of consecutive slots (entries) of its own, so per step the warp multiplies R
+// rows of B, one per group.  Groups are independent -- own slots, own row changes, own sum -- so a
+// flush needs no sum over the warp and a row may end at any step.  The rows of B land in a ring of
+// eight steps in shared memory, filled by cp.async; columns, values and row changes of G steps (a
+// strip) are staged by the group's lanes, one slot each.
 //
-// What bounds it: the L2 hands a streaming multiprocessor about 30 bytes per clock of scattered
-// 128-byte rows (42 of 512-byte rows), and the ring keeps enough of them in flight to be there.
+// What bounds it: instructions.  On 6.8 M entries a walk of one row (128 features) per warp and step
+// takes 275 us, of two rows of 64 features 182 us, of four rows of 32 features 128 us: the time goes
+// down with the bytes at 17 TB/s and with the steps not at all, because the work per row that does not
+// depend on its length (its address, its row change, its share of staging and of the flush) stays.
+// Everything below is written for that share:
+//   * two chunks per lane (CH = 2), so that half the lanes carry a row and the other half another one;
+//   * columns, row changes and values are read four steps at a time; a row change is the row id
+//     itself in the slot where the row starts, -1 elsewhere, so that it needs neither masks nor a second
+//     look-up; values are staged as pairs for the two-wide FMA;
+//   * only copies and the write-out look at whether a lane has features; sums of lanes that have none
+//     run on whatever the ring holds and are dropped;
+//   * whether a row may also be held by another group is decided once for the first and once for the
+//     last row of a walk.
 //
-// ODD is the form for operands without 16-byte alignment (feature counts, leading dimensions or
-// bases that are no multiple of four floats).  A row of B then starts at any word: the group copies
-// the aligned 16-byte chunks that cover it -- every chunk holds at least one word of the row, so it
-// never leaves the 16-byte granule, hence the page, of valid memory -- and reads its features back
-// word by word behind the row's shift of 0..3 words.  A lane owns features gl + G * v; which v it
-// takes first is rotated by the group so that the groups of a warp read different banks.
+// SH is the form for operands without 16-byte alignment (feature counts, leading dimensions or bases
+// that are no multiple of four floats).  A row of B then starts at any word: the group copies the
+// aligned 16-byte chunks that cover it -- each of them holds at least one word of the row, so it never
+// leaves the 16-byte granule, hence the page, of valid memory -- and reads its features back word by
+// word behind the row's shift of 0..3 words.  A lane owns features gl + G * v; which v it takes first
+// is rotated by the group so that the groups of a warp read different banks.
 #pragma once
 
 #include "lf_spmm_gather.cuh"
 
 namespace lf {
 
-constexpr int kGroupSteps = 16;                                                      // steps in flight
-template <int G> constexpr int kGroupStrips = (kGroupSteps + G - 1) / G + 1;         // strips held: those ahead and the one in use
-template <int G> constexpr int kGroupOddFeatures = 4 * G - 4;                        // features per group behind any shift
+constexpr int kGroupSteps = 8;   // steps in flight: two commit groups of four
+constexpr unsigned kAllLanes = 0xffffffffu;
 
-// Lanes per group for N features and the number of times the slots are walked for it (blocks along y).
-// Operands with 16-byte alignment: the smallest group that holds a row of B, 32 lanes from 128 features
-// on.  Others: a group of G lanes takes 4 G - 4 features; the walk itself costs about a fifth of the
-// multiplication by a full warp (staging, addresses), the rest goes down with the rows per step.
-struct GroupCfg { int G, passes; };
-inline GroupCfg pick_group(bool aligned, int N) {
-  if (aligned) {
-    const int G = N <= 32 ? 8 : (N <= 64 ? 16 : 32);
-    return {G, (N + 4 * G - 1) / (4 * G)};
-  }
-  GroupCfg best{32, 0};
+template <int G> constexpr int kGroupStrips = G == 4 ? 4 : 2;   // strips held: those being copied and the one in use
+
+// Lanes per group, chunks per lane and the number of walks (blocks along y) for N features.
+struct GroupCfg { int G, CH, passes; };
+// 16-byte aligned rows of `vec` features per chunk: groups as narrow as the row, two chunks per
+// lane for rows of more than 128 bytes.
+inline GroupCfg pick_group(int N, int vec) {
+  if (N <= 4 * vec) return {4, 1, 1};
+  if (N <= 8 * vec) return {8, 1, 1};
+  if (N <= 16 * vec) return {8, 2, 1};
+  if (N <= 32 * vec) return {16, 2, 1};
+  return {32, 2, (N + 64 * vec - 1) / (64 * vec)};
+}
+// Shifted rows: a group of G lanes takes 4 G - 4 features behind any shift; a third of a full warp's
+// time per walk is work that fewer lanes do not save.
+inline GroupCfg pick_group_shifted(int N) {
+  GroupCfg best{32, 1, 0};
   float cheapest = 0.f;
-  for (int G = 32; G >= 8; G >>= 1) {
+  for (int G = 32; G >= 4; G >>= 1) {
     const int passes = (N + 4 * G - 5) / (4 * G - 4);
-    const float cost = passes * (0.2f + G / 32.f);
+    const float cost = passes * (0.35f + 0.65f * G / 32.f);
     if (!best.passes || cost < cheapest) {
-      best = {G, passes};
+      best = {G, 1, passes};
       cheapest = cost;
     }
   }
   return best;
 }
+template <int G, int CH, int VEC, bool SH> constexpr int kGroupFeatures = SH ? 4 * G - 4 : G * CH * VEC;
 
-// Shared memory of one warp: the ring (a few words longer, because a shifted read of features past the
-// row's end is not masked), then columns, values and row ids of the strips, then the shifts.
-template <int G, bool ODD>
+// Shared memory of one warp: the ring, then value pairs, columns and row starts of the strips, then
+// (SH) the shifts in bytes and a few words that a shifted read past the row's end may touch.
+template <int G, int CH, bool SH>
 struct GroupSmem {
-  static constexpr int kStrip = kGroupStrips<G> * 32;
-  static constexpr int kBytes = kGroupSteps * 512 + (ODD ? 16 : 0) + kStrip * 12 + (ODD ? kStrip : 0);
+  static constexpr int kCells = kGroupStrips<G> * 32;
+  static constexpr int kRing = kGroupSteps * CH * 512;
+  static constexpr int kBytes = kRing + kCells * 16 + (SH ? kCells * 4 + 16 : 0);
   static_assert(kBytes % 16 == 0, "the next warp's ring starts on a 16-byte boundary");
 };
+
+// place of step q (0 .. G-1) of group g inside a strip: four steps of a group are adjacent
+template <int G>
+__device__ __forceinline__ int group_cell(int q, int g) { return (q >> 2) * (4 * (32 / G)) + g * 4 + (q & 3); }
 
 // Row ids of the slots of one bucket: slot i belongs to ELL row i >> wlog.
 template <int G>
 struct EllRowIds {
   const int32_t* __restrict__ rows;   // of the group's first ELL row
   int wlog, n;                        // log2(width), slots of the group
-  int first, last;
-  bool head_open, tail_open, all_open;
-  int pr, carry;
+  int first, pr, carry;
+  bool head_open, tail_open;
 
-  __device__ __forceinline__ void init(const int32_t* bucket_rows, int wlog_, int64_t e0, int64_t e1, int64_t ell_rows,
-                                       bool all) {
+  __device__ __forceinline__ void init(const int32_t* bucket_rows, int wlog_, int64_t e0, int64_t e1, int64_t ell_rows) {
     rows = bucket_rows + e0;
     wlog = wlog_;
     n = e1 > e0 ? (int)((e1 - e0) << wlog_) : 0;
-    all_open = all;
-    first = last = 0;
+    first = pr = 0;
     head_open = tail_open = false;
     if (n > 0) {
       first = bucket_rows[e0];
-      last = bucket_rows[e1 - 1];
       head_open = e0 > 0 && bucket_rows[e0 - 1] == first;
-      tail_open = e1 < ell_rows && bucket_rows[e1] == last;
+      tail_open = e1 < ell_rows && bucket_rows[e1] == bucket_rows[e1 - 1];
     }
     carry = first;
-    pr = 0;
   }
   __device__ __forceinline__ void prefetch(int k, int gl) {
     if (n > 0) pr = rows[min(k * G + gl, n - 1) >> wlog];
   }
-  // writes the row ids of strip k; bit (lane) of the result: that slot carries another row than the one before
-  __device__ __forceinline__ uint32_t stage(int, int32_t* rd, int gl) {
-    rd[gl] = pr;
-    int before = __shfl_up_sync(0xffffffffu, pr, 1, G);
+  __device__ __forceinline__ void stage(int, int32_t* rd, int g, int gl) {
+    int before = __shfl_up_sync(kAllLanes, pr, 1, G);
     if (gl == 0) before = carry;
-    carry = __shfl_sync(0xffffffffu, pr, G - 1, G);
-    return __ballot_sync(0xffffffffu, pr != before);
+    rd[group_cell<G>(gl, g)] = pr != before ? pr : -1;
+    carry = __shfl_sync(kAllLanes, pr, G - 1, G);
   }
-  __device__ __forceinline__ int first_row() const { return first; }
-  // may another group hold a part of this row?
-  __device__ __forceinline__ bool open(int row, bool /*at_end*/) const {
-    return all_open || (row == first && head_open) || (row == last && tail_open);
-  }
-  __device__ __forceinline__ void finish() {}
+  __device__ __forceinline__ bool last_open() const { return tail_open; }
 };
 
 // Rows of consecutive CSR entries.  Lane gl watches the start of row r + 1 + gl, r being the row the
-// walk has reached; starts that fall into a strip become bits, the rows they start their ids.
+// walk has reached; a start that falls into a strip puts the row's number into its slot.
 template <int G>
 struct CsrRowIds {
   const int64_t* __restrict__ indptr;   // of the first row of the range
   int64_t origin;                       // entry the group starts with
-  int64_t num_rows;
-  int n;
-  int64_t r;
-  int first, nb;
-  bool head_open, tail_open;
+  int num_rows, n, r, first, nb;
+  bool head_open;
 
-  __device__ __forceinline__ int start_of(int64_t row) const {   // relative to the group's first entry, saturated
-    const int64_t d = indptr[row < num_rows ? row : num_rows] - origin;
+  __device__ __forceinline__ int start_of(int row) const {   // relative to the group's first entry, saturated
+    const int64_t d = indptr[min(row, num_rows)] - origin;
     return d > 0x3fffffff ? 0x3fffffff : (int)d;
   }
+  static __device__ __forceinline__ int count(bool mine, int g) {   // lanes of the group with `mine`
+    const uint32_t m = __ballot_sync(kAllLanes, mine);
+    return __popc(G == 32 ? m : (m >> (g * G)) & ((1u << (G % 32)) - 1u));
+  }
   // entries [s0, s1) of the range whose first entry is `base`; every lane of the warp takes part
-  __device__ __forceinline__ void init(const int64_t* range_indptr, int64_t rows, int64_t base, int64_t s0, int64_t s1, int lane) {
-    constexpr unsigned kAll = 0xffffffffu;
-    const int gl = lane % G, shift = lane / G * G;
+  __device__ __forceinline__ void init(const int64_t* range_indptr, int rows, int64_t base, int64_t s0, int64_t s1, int g, int gl) {
     indptr = range_indptr;
     num_rows = rows;
     n = s1 > s0 ? (int)(s1 - s0) : 0;
     origin = base + s0;
-    int64_t lo = 0, hi = n > 0 ? rows : 1;   // indptr[lo] <= origin, answer in [lo, hi): one probe per lane and round
-    while (__any_sync(kAll, hi - lo > 1)) {
-      const int64_t span = hi - lo;
-      int64_t q = lo + ((int64_t)(gl + 1) * span) / (G + 1);
+    int lo = 0, hi = n > 0 ? rows : 1;   // indptr[lo] <= origin, answer in [lo, hi): one probe per lane and round
+    while (__any_sync(kAllLanes, hi - lo > 1)) {
+      const int span = hi - lo;
+      int q = lo + (int)(((int64_t)(gl + 1) * span) / (G + 1));
       if (q <= lo) q = lo + 1;
-      const bool le = span > 1 && indptr[q] <= origin;
-      const uint32_t m = __ballot_sync(kAll, le) >> shift;
-      const int cnt = __popc(G == 32 ? m : m & ((1u << (G % 32)) - 1u));   // probes are monotone
-      const int64_t qlo = __shfl_sync(kAll, q, cnt > 0 ? cnt - 1 : 0, G);
-      const int64_t qhi = __shfl_sync(kAll, q, cnt < G ? cnt : G - 1, G);
+      const int cnt = count(span > 1 && indptr[q] <= origin, g);   // probes are monotone
+      const int qlo = __shfl_sync(kAllLanes, q, cnt > 0 ? cnt - 1 : 0, G);
+      const int qhi = __shfl_sync(kAllLanes, q, cnt < G ? cnt : G - 1, G);
       if (span > 1) {
         if (cnt > 0) lo = qlo;
         if (cnt < G) hi = qhi;
       }
     }
-    r = lo;
-    first = (int)lo;
+    first = r = lo;
     head_open = n > 0 && indptr[lo] < origin;
-    tail_open = false;
     nb = 0x3fffffff;
   }
   __device__ __forceinline__ void prefetch(int, int gl) {
     if (n > 0) nb = start_of(r + 1 + gl);
   }
-  __device__ __forceinline__ uint32_t stage(int k, int32_t* rd, int gl) {
-    constexpr unsigned kAll = 0xffffffffu;
+  __device__ __forceinline__ void stage(int k, int32_t* rd, int g, int gl) {
     const int lo = k * G, hi = min(lo + G, n);
-    const int shift = (threadIdx.x & 31) / G * G;
-    uint32_t starts = 0;
+    rd[group_cell<G>(gl, g)] = -1;
     for (;;) {
-      const bool in = nb < hi;
-      const int after = __shfl_down_sync(kAll, nb, 1, G);
-      if (in && (gl == G - 1 || after != nb)) rd[nb - lo] = (int)(r + 1 + gl);   // of empty rows in between the last one counts
-      starts |= __reduce_or_sync(kAll, in ? 1u << (shift + nb - lo) : 0u);
-      const uint32_t m = __ballot_sync(kAll, in) >> shift;
-      const int cnt = __popc(G == 32 ? m : m & ((1u << (G % 32)) - 1u));
-      r += cnt;
-      if (!__any_sync(kAll, cnt == G)) break;   // all G watched starts passed: there may be more (many short rows)
       __syncwarp();
+      const bool in = nb < hi;
+      const int after = __shfl_down_sync(kAllLanes, nb, 1, G);
+      if (in && (gl == G - 1 || after != nb)) rd[group_cell<G>(nb - lo, g)] = r + 1 + gl;   // of empty rows in between the last one counts
+      const int cnt = count(in, g);
+      r += cnt;
+      if (!__any_sync(kAllLanes, cnt == G)) break;   // all G watched starts passed: there may be more (many short rows)
       prefetch(k, gl);
     }
-    return starts;
   }
-  __device__ __forceinline__ int first_row() const { return first; }
-  __device__ __forceinline__ bool open(int row, bool at_end) const {
-    return (row == first && head_open) || (at_end && tail_open);
-  }
-  __device__ __forceinline__ void finish() {
-    if (n > 0) tail_open = start_of(r + 1) > n;
-  }
+  __device__ __forceinline__ bool last_open() const { return start_of(r + 1) > n; }
 };
 
-// Sums and write-out of one group's row: VEC features per lane, or four single words per lane (ODD).
-template <int G, int VEC, bool ODD>
+__device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ float2 as_floats(uint64_t v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ uint64_t as_pair(uint32_t lo, uint32_t hi) {
+  uint64_t v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(lo), "r"(hi));
+  return v;
+}
+
+// The sum of one row, and its way to C.
+template <int G, int CH, int VEC, bool SH>
 struct GroupSum {
-  Chunk<VEC> acc;
-  __device__ __forceinline__ void zero() { acc.zero(); }
-  __device__ __forceinline__ void write(float* row, int gl, int, int nf, bool open) const {
-    if (gl * VEC < nf) {
-      if (open) acc.red(row + gl * VEC); else acc.store_stream(row + gl * VEC);
+  static constexpr int kPairs = CH * VEC / 2;
+  uint64_t a[kPairs];
+  __device__ __forceinline__ void zero() {
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) a[i] = 0;
+  }
+  // x: this lane's first chunk of the row in the ring (CH chunks, 512 bytes apart)
+  __device__ __forceinline__ void add(uint64_t val, const unsigned char* x) {
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      if constexpr (VEC == 4) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(x + c * 512);
+        a[2 * c] = fma_pair(val, v.x, a[2 * c]);
+        a[2 * c + 1] = fma_pair(val, v.y, a[2 * c + 1]);
+      } else {
+        const uint4 v = *reinterpret_cast<const uint4*>(x + c * 512);
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)   // a bf16 is the upper half of the float with the same value
+          a[4 * c + i] = fma_pair(val, as_pair(w[i] << 16, w[i] & 0xffff0000u), a[4 * c + i]);
+      }
     }
   }
-};
-template <int G, int VEC>
-struct GroupSum<G, VEC, true> {
-  float a[4];
-  __device__ __forceinline__ void zero() { a[0] = a[1] = a[2] = a[3] = 0.f; }
-  static __device__ __forceinline__ int feature(int v, int gl, int g) { return gl + G * ((v + g) & 3); }
-  __device__ __forceinline__ void write(float* row, int gl, int g, int nf, bool open) const {
+  // row: this lane's first feature in C; nf: features from there to the end of the row
+  __device__ __forceinline__ void write(float* row, int nf, bool open) const {
 #pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int f = feature(v, gl, g);
-      if (f < nf) {
-        if (open) atomicAdd(row + f, a[v]); else __stcs(row + f, a[v]);
+    for (int c = 0; c < CH; ++c) {
+      if (c * G * VEC < nf) {
+#pragma unroll
+        for (int h = 0; h < VEC / 4; ++h) {
+          float* p = row + c * G * VEC + 4 * h;
+          const uint64_t lo = a[c * VEC / 2 + 2 * h], hi = a[c * VEC / 2 + 2 * h + 1];
+          if (open) {
+            const float2 x = as_floats(lo), y = as_floats(hi);
+            red_add_v4(p, x.x, x.y, y.x, y.y);
+          } else {
+            __stcs(reinterpret_cast<ulonglong2*>(p), make_ulonglong2(lo, hi));
+          }
+        }
       }
     }
   }
 };
+template <int G, int VEC>
+struct GroupSum<G, 1, VEC, true> {
+  float a[4];
+  __device__ __forceinline__ void zero() { a[0] = a[1] = a[2] = a[3] = 0.f; }
+  // feature v of lane gl: the groups that share banks (G = 4: every other one) start with different v
+  static __device__ __forceinline__ int feature(int v, int g, int gl) { return gl + G * ((v + (G == 4 ? g >> 1 : g)) & 3); }
+};
 
 // One warp; cols / vals point at the calling group's first slot (vals == nullptr: all ones), `ids`
 // knows the rows of its ids.n slots (0: the group has nothing to do).  WC: row changes happen only at
-// multiples of WC slots.  C: row 0 of the output the row ids count from, at feature f0.
-template <int G, int VEC, bool ODD, int WC, class Rows>
-__device__ __forceinline__ void walk_group_ring(Rows& ids, const int32_t* __restrict__ cols, const float* __restrict__ vals,
+// multiples of WC slots.  all_open: every row may be held by other groups too.  C: row 0 of the output
+// the row ids count from, at the first feature of this walk; nf: features from there on.
+template <int G, int CH, int VEC, bool SH, int WC, class Rows>
+__device__ __forceinline__ void walk_group_ring(Rows& ids, bool all_open, const int32_t* __restrict__ cols,
+                                                const float* __restrict__ vals,
                                                 const typename BTraits<VEC>::elem* __restrict__ B, int ldb,
-                                                float* __restrict__ C, int64_t ldc, int nf, int lane, unsigned char* smem) {
-  constexpr unsigned kAll = 0xffffffffu;
-  constexpr int U = 8, D = kGroupSteps, NB = kGroupStrips<G>, kStrip = GroupSmem<G, ODD>::kStrip;
-  static_assert(D == 2 * U && G % U == 0 && U % WC == 0, "two commit groups of eight steps in flight");
-  static_assert(!ODD || VEC == 4, "the shifted form is for float32 rows");
-  const int gl = lane % G, g = lane / G;
-  uint32_t* so = reinterpret_cast<uint32_t*>(smem + D * 512 + (ODD ? 16 : 0));
-  float* sv = reinterpret_cast<float*>(so + kStrip);
-  int32_t* rd = reinterpret_cast<int32_t*>(sv + kStrip);
-  uint8_t* ss = reinterpret_cast<uint8_t*>(rd + kStrip);
+                                                float* __restrict__ C, int64_t ldc, int nf, int g, int gl,
+                                                unsigned char* smem) {
+  using Elem = typename BTraits<VEC>::elem;
+  using Smem = GroupSmem<G, CH, SH>;
+  constexpr int U = 4, R = 32 / G, kCells = Smem::kCells, kHalf = U * CH * 512;
+  static_assert(kGroupSteps == 2 * U && G % U == 0, "two commit groups of four steps in flight");
+  static_assert(!SH || (VEC == 4 && CH == 1), "the shifted form is for float32 rows, one chunk per lane");
+  uint64_t* sv = reinterpret_cast<uint64_t*>(smem + Smem::kRing);   // {value, value}
+  uint32_t* so = reinterpret_cast<uint32_t*>(sv + kCells);          // column or kNoGather
+  int32_t* rd = reinterpret_cast<int32_t*>(so + kCells);            // row that starts here, or -1
+  uint32_t* ss = reinterpret_cast<uint32_t*>(rd + kCells);          // SH: bytes between chunk and row start
+  const int lane = g * G + gl;
   const int n = ids.n;
-  const int nmax = __reduce_max_sync(kAll, n);
+  const int nmax = __reduce_max_sync(kAllLanes, n);
   const int nstrips = (nmax + G - 1) / G;
-  const bool active = ODD || gl * VEC < nf;
-  GroupSum<G, VEC, ODD> sum;
+
+  // where this lane's chunks lie in a row, and whether they hold features (lanes past the last feature
+  // copying its last chunk again took 237 us, masking them 181 us, on 3.7 M entries, 100 features)
+  const char* Bl = reinterpret_cast<const char*>(B) + (SH ? 0 : gl * 16);
+  const bool in1 = SH || gl * VEC < nf, in2 = CH == 2 && (gl + G) * VEC < nf;
+  const uint32_t pitch = (uint32_t)ldb * (uint32_t)sizeof(Elem), pitch_c = (uint32_t)ldc * 4u;   // checked by the launch
+  const int over = SH ? gl * 16 - nf * 4 : 0;   // SH: chunk gl is needed while the shift is larger than this
+
+  GroupSum<G, CH, VEC, SH> sum;
   sum.zero();
-  int cur = ids.first_row();
-  auto flush = [&](int row, bool at_end) {
-    sum.write(C + (int64_t)row * ldc, gl, g, nf, ids.open(row, at_end));
+  int cur = ids.first;
+  bool open = all_open || ids.head_open;
+  float* Cl = C + (SH ? 0 : gl * VEC);
+  auto flush = [&](bool open_now) {
+    float* row = reinterpret_cast<float*>(const_cast<void*>(row_of_b(Cl, (uint32_t)cur, pitch_c)));
+    if constexpr (SH) {
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int f = sum.feature(v, g, gl);
+        if (f < nf) {
+          if (open_now) atomicAdd(row + f, sum.a[v]); else __stcs(row + f, sum.a[v]);
+        }
+      }
+    } else {
+      sum.write(row, nf - gl * VEC, open_now);
+    }
     sum.zero();
   };
 
@@ -245,114 +304,94 @@ __device__ __forceinline__ void walk_group_ring(Rows& ids, const int32_t* __rest
     pv = in ? (vals ? __ldcs(vals + i) : 1.f) : 0.f;
     ids.prefetch(k, gl);
   };
-  uint32_t chg[NB];   // per strip held: bit (lane) = that slot starts another row
-#pragma unroll
-  for (int b = 0; b < NB; ++b) chg[b] = 0;
-  const uint32_t base_shift = (uint32_t)(reinterpret_cast<uintptr_t>(B) >> 2);
-  auto store_strip = [&](int k, int at) {
-    const int cell = at * 32 + lane;
+  const int my_cell = group_cell<G>(gl, g);
+  auto store_strip = [&](int k, int base) {
+    const int cell = base + my_cell;
     so[cell] = pv != 0.f ? (uint32_t)pc : kNoGather;
-    sv[cell] = pv;
-    if constexpr (ODD) ss[cell] = (uint8_t)((base_shift + (uint32_t)pc * (uint32_t)ldb) & 3u);
-    const uint32_t m = ids.stage(k, rd + at * 32 + g * G, gl);
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-      if (b == at) chg[b] = m;
+    sv[cell] = as_pair(__float_as_uint(pv), __float_as_uint(pv));
+    if constexpr (SH) ss[cell] = ((uint32_t)reinterpret_cast<uintptr_t>(B) + (uint32_t)pc * pitch) & 12u;
+    ids.stage(k, rd + base, g, gl);
   };
-  int in_at = 0;   // place of the newest strip
   load_strip(0);
   store_strip(0, 0);
   __syncwarp();
   if (nstrips > 1) load_strip(1);
 
-  const float4* ring_lane = reinterpret_cast<const float4*>(smem) + lane;
-  const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring_lane);
-  const uint32_t pitch = (uint32_t)ldb * (uint32_t)sizeof(typename BTraits<VEC>::elem);   // checked by the launch
-  const typename BTraits<VEC>::elem* __restrict__ Bl = ODD ? B : B + gl * VEC;
-  const uint4* so4 = reinterpret_cast<const uint4*>(so);
-  const float4* sv4 = reinterpret_cast<const float4*>(sv);
-  auto issue_batch = [&](int j0, auto slot_tag) {
-    constexpr int SLOT = decltype(slot_tag)::value;
-    if (j0 < nstrips * G) {
-      const int q0 = j0 % G;
-      if (q0 == 0 && j0 > 0) {   // first steps of a strip: it moves from registers to shared memory
-        const int k = j0 / G;    // (its place held a strip that has been added up)
-        in_at = in_at + 1 == NB ? 0 : in_at + 1;
+  const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(smem) + lane * 16;
+  int k_next = 1, in_cell = 0, in_half = 0;   // producer: next strip to store, place in the strips, half of the ring
+  // start the copies of four steps and close them as one group; past the end the group is empty, which
+  // keeps the number of groups per batch constant
+  auto issue_batch = [&](int j) {
+    if (j < nstrips * G) {
+      if ((in_cell & 31) == 0 && j > 0) {   // first steps of a strip: it moves from registers to shared memory
+        __syncwarp();                       // (its place held a strip that has been added up)
+        store_strip(k_next, in_cell);
         __syncwarp();
-        store_strip(k, in_at);
-        __syncwarp();
-        if (k + 1 < nstrips) load_strip(k + 1);
+        if (++k_next < nstrips) load_strip(k_next);
       }
-      const int at = in_at * 32 + g * G + q0;
-      const uint4 oa = so4[at >> 2], ob = so4[(at >> 2) + 1];
-      const uint32_t o[U] = {oa.x, oa.y, oa.z, oa.w, ob.x, ob.y, ob.z, ob.w};
+      const uint4 o4 = *reinterpret_cast<const uint4*>(so + in_cell + g * 4);
+      const uint32_t o[U] = {o4.x, o4.y, o4.z, o4.w};
+      const uint32_t dst = ring_s + in_half;
+      if constexpr (SH) {
+        const int4 h4 = *reinterpret_cast<const int4*>(ss + in_cell + g * 4);
+        const int h[U] = {h4.x, h4.y, h4.z, h4.w};
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if constexpr (ODD) {
-          if (o[u] != kNoGather) {
-            const uint64_t a = reinterpret_cast<uint64_t>(row_of_b(Bl, o[u], pitch));
-            if (gl * 4 < (int)((a >> 2) & 3) + nf)
-              cp_async_16(ring_s + (uint32_t)(SLOT + u) * 512u, reinterpret_cast<const void*>((a & ~15ull) + gl * 16));
-          }
-        } else {
-          if (o[u] != kNoGather && active) cp_async_16(ring_s + (uint32_t)(SLOT + u) * 512u, row_of_b(Bl, o[u], pitch));
+        for (int u = 0; u < U; ++u)
+          if (o[u] != kNoGather && h[u] > over)
+            cp_async_16(dst + u * 512, reinterpret_cast<const void*>((reinterpret_cast<uint64_t>(row_of_b(Bl, o[u], pitch)) & ~15ull) + gl * 16));
+      } else {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const char* src = reinterpret_cast<const char*>(row_of_b(Bl, o[u], pitch));
+          if (o[u] != kNoGather && in1) cp_async_16(dst + u * (CH * 512), src);
+          if (CH == 2 && o[u] != kNoGather && in2) cp_async_16(dst + u * (CH * 512) + 512, src + G * 16);
         }
       }
+      in_cell = (in_cell + U * R) & (kCells - 1);
+      in_half ^= kHalf;
     }
     cp_async_commit();
   };
-  issue_batch(0, std::integral_constant<int, 0>{});
-  issue_batch(U, std::integral_constant<int, U>{});
+  issue_batch(0);
+  issue_batch(U);
   wait_for_prior_grid();   // no store or atomic to C before the row-clearing launch is complete
 
-  int out_at = 0;          // place of the strip being added up
-  auto add_batch = [&](int jc, auto slot_tag) {
-    constexpr int SLOT = decltype(slot_tag)::value;
-    const int q0 = jc % G;
-    if (q0 == 0 && jc > 0) out_at = out_at + 1 == NB ? 0 : out_at + 1;
-    const int at = out_at * 32 + g * G + q0;
-    const float4 va = sv4[at >> 2], vb = sv4[(at >> 2) + 1];
-    const float val[U] = {va.x, va.y, va.z, va.w, vb.x, vb.y, vb.z, vb.w};
-    uint32_t m = chg[0];
-#pragma unroll
-    for (int b = 1; b < NB; ++b)
-      if (b == out_at) m = chg[b];
-    const uint32_t starts = m >> (g * G + q0);
-    uint2 shifts = make_uint2(0u, 0u);
-    if constexpr (ODD) shifts = *reinterpret_cast<const uint2*>(ss + at);
-    cp_async_wait<1>();            // all but the newest group of copies have landed
-    if constexpr (ODD) __syncwarp();   // lanes read words that other lanes copied
+  int cell = g * 4, half = 0;   // consumer
+  for (int j = 0; j < nmax; j += U) {
+    const int4 r4 = *reinterpret_cast<const int4*>(rd + cell);
+    const ulonglong2 va = *reinterpret_cast<const ulonglong2*>(sv + cell), vb = *reinterpret_cast<const ulonglong2*>(sv + cell + 2);
+    const int start[U] = {r4.x, r4.y, r4.z, r4.w};
+    const uint64_t val[U] = {va.x, va.y, vb.x, vb.y};
+    int4 h4 = make_int4(0, 0, 0, 0);
+    if constexpr (SH) h4 = *reinterpret_cast<const int4*>(ss + cell);
+    const int h[U] = {h4.x, h4.y, h4.z, h4.w};
+    cp_async_wait<1>();                // all but the newest group of copies have landed
+    if constexpr (SH) __syncwarp();    // lanes read words that other lanes copied
+    const unsigned char* x = smem + half + (SH ? g * G * 16 : lane * 16);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      if (u % WC == 0 && ((starts >> u) & 1u)) {
-        flush(cur, false);
-        cur = rd[at + u];
+      if (u % WC == 0 && start[u] >= 0) {
+        flush(open);
+        cur = start[u];
+        open = all_open;
       }
-      if (val[u] != 0.f && active) {
-        if constexpr (ODD) {
-          const uint32_t sh = ((u < 4 ? shifts.x : shifts.y) >> (8 * (u & 3))) & 3u;
-          const float* x = reinterpret_cast<const float*>(smem) + (SLOT + u) * 128 + g * G * 4 + sh;
+      if constexpr (SH) {
+        const float v0 = as_floats(val[u]).x;
+        if (v0 != 0.f) {
+          const unsigned char* w = x + u * 512 + h[u];
 #pragma unroll
-          for (int v = 0; v < 4; ++v) sum.a[v] = fmaf(val[u], x[sum.feature(v, gl, g)], sum.a[v]);
-        } else {
-          typename BTraits<VEC>::raw x;
-          const float4 raw = ring_lane[(SLOT + u) * 32];
-          if constexpr (VEC == 8) x.v = make_uint4(__float_as_uint(raw.x), __float_as_uint(raw.y), __float_as_uint(raw.z), __float_as_uint(raw.w));
-          else x.v = raw;
-          chunk_fma(sum.acc, val[u], x);
+          for (int v = 0; v < 4; ++v) sum.a[v] = fmaf(v0, *reinterpret_cast<const float*>(w + sum.feature(v, g, gl) * 4), sum.a[v]);
         }
+      } else {
+        if (as_floats(val[u]).x != 0.f) sum.add(val[u], x + u * (CH * 512));
       }
     }
-    if constexpr (ODD) __syncwarp();   // every lane has read before the slots are refilled
-    issue_batch(jc + D, slot_tag);     // refills exactly the ring slots read above
-  };
-  for (int jc0 = 0; jc0 < nmax; jc0 += D) {
-    add_batch(jc0, std::integral_constant<int, 0>{});
-    if (jc0 + U >= nmax) break;
-    add_batch(jc0 + U, std::integral_constant<int, U>{});
+    if constexpr (SH) __syncwarp();    // every lane has read before the slots are refilled
+    cell = (cell + U * R) & (kCells - 1);
+    half ^= kHalf;
+    issue_batch(j + 2 * U);            // refills exactly the ring slots read above
   }
-  ids.finish();
-  if (n > 0) flush(cur, true);
+  if (n > 0) flush(open || ids.last_open());
 }
 
 }  // namespace lf
