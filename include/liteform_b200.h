@@ -127,6 +127,10 @@ int lf_hyb_stats(const int64_t* indptr /*[dev] M+1*/, const int32_t* indices /*[
                  int64_t num_rows, int64_t num_cols, int32_t num_parts,
                  int64_t* class_stats /*[dev] P*11*3*/, int64_t* colmask_hist /*[dev] P*2048*/,
                  void* workspace /*[dev]*/, size_t workspace_bytes, void* stream);
+/* Turns such a histogram, in place, into counts per SET of classes: colmask_hist[p*2048 + c] becomes the
+ * number of columns of partition p that at least one class of the bit set c touches, which is
+ * len(col_indices) of a bucket merged from the classes c. */
+int lf_hyb_class_coverage(int64_t* colmask_hist /*[dev] P*2048*/, int32_t num_parts, void* stream);
 
 /* ---------------------------------------------------------------------------------------------
  * lf_hyb_stats without any workspace argument.  It has no counterpart in the reference; it is

@@ -74,6 +74,7 @@ SIGNATURES = {
     "lf_csr_validate": (C.c_int, [vp, vp, C.c_int64, C.c_int64, C.c_int64, vp]),
     "lf_hyb_stats_workspace_bytes": (C.c_size_t, [C.c_int64, C.c_int64, C.c_int32]),
     "lf_hyb_stats": (C.c_int, [vp, vp, C.c_int64, C.c_int64, C.c_int32, vp, vp, vp, C.c_size_t, vp]),
+    "lf_hyb_class_coverage": (C.c_int, [vp, C.c_int32, vp]),
     "lf_hyb_stats_static": (C.c_int, [vp, vp, C.c_int64, C.c_int64, C.c_int32, vp, vp, vp]),
     "lf_hyb_build_workspace_bytes": (C.c_size_t, [C.c_int64, C.c_int64, C.c_int32, C.c_int32]),
     "lf_hyb_fill_scratch_bytes": (C.c_size_t, [C.c_int64]),

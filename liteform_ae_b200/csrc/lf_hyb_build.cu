@@ -7,6 +7,9 @@
 //
 // None of the kernels below waits on another thread block: offsets across blocks come from a
 // separate scan launch, never from a look-back spin.
+#include <stdlib.h>
+#include <string.h>
+
 #include <mutex>
 
 #include "lf_common.cuh"
@@ -401,6 +404,28 @@ colmask_hist_kernel(const uint32_t* __restrict__ colmask, int64_t num_cols, int6
     if (s_hist[i]) atomicAdd(hist + (size_t)p * LF_COLMASK_BINS + i, (unsigned long long)s_hist[i]);
 }
 
+// In place, one thread block per partition: histogram over class masks -> for every set of classes the
+// number of columns that a class of the set touches.  f[S] = columns whose mask lies inside S comes from
+// 11 rounds of pairwise sums (for every S at once), and the columns that miss c are f[complement of c].
+// The width search reads about 20 sets per partition; summing the bins of each on the host took 350 of
+// the 465 us of a search, these rounds take 3 us.
+__global__ void __launch_bounds__(512)
+class_coverage_kernel(unsigned long long* __restrict__ hist) {
+  __shared__ unsigned long long f[LF_COLMASK_BINS];
+  unsigned long long* h = hist + (size_t)blockIdx.x * LF_COLMASK_BINS;
+  for (int i = threadIdx.x; i < LF_COLMASK_BINS; i += blockDim.x) f[i] = h[i];
+  for (int bit = 1; bit < LF_COLMASK_BINS; bit <<= 1) {
+    __syncthreads();
+    for (int q = threadIdx.x; q < LF_COLMASK_BINS / 2; q += blockDim.x) {
+      const int i = ((q & ~(bit - 1)) << 1) | (q & (bit - 1));   // the q-th set without `bit`
+      f[i | bit] += f[i];
+    }
+  }
+  __syncthreads();
+  const unsigned long long all = f[LF_COLMASK_BINS - 1];
+  for (int i = threadIdx.x; i < LF_COLMASK_BINS; i += blockDim.x) h[i] = all - f[LF_COLMASK_BINS - 1 - i];
+}
+
 // ------------------------------------------------------------------------------------------
 // plan / fill
 // ------------------------------------------------------------------------------------------
@@ -468,7 +493,8 @@ hyb_count_kernel(const int64_t* __restrict__ indptr, const int32_t* __restrict__
 // blockIdx.x = category; exclusive scan of that category's per-block counts over all blocks.
 __global__ void __launch_bounds__(256)
 scan_blocks_kernel(const int32_t* __restrict__ block_counts, int64_t num_blocks, int ncat,
-                   int64_t* __restrict__ block_offsets, int64_t* __restrict__ totals) {
+                   int64_t* __restrict__ block_offsets, int64_t* __restrict__ totals, const int32_t* __restrict__ err,
+                   const int64_t* __restrict__ last_ptr) {
   __shared__ int s_scan[256 / 32 + 1];
   const int cat = blockIdx.x;
   int64_t running = 0;
@@ -481,6 +507,10 @@ scan_blocks_kernel(const int32_t* __restrict__ block_counts, int64_t num_blocks,
     running += tot;
   }
   if (threadIdx.x == 0) totals[cat] = running;
+  if (cat == 0 && threadIdx.x == 0) {   // what the host wants to know besides, for one read-back
+    totals[ncat] = *err;
+    totals[ncat + 1] = *last_ptr;
+  }
 }
 
 // One thread per matrix row.  Writes, for every ELL row the matrix row produces: the row id, and
@@ -725,16 +755,25 @@ BuildWs carve_build(void* base, int64_t rows, int num_parts, int nb) {
   BuildWs w;
   w.pbo = (int32_t*)take(sizeof(int32_t) * (num_parts + 1));
   w.widths = (int32_t*)take(sizeof(int32_t) * (nb > 0 ? nb : 1));
+  w.err = (int32_t*)take(sizeof(int32_t) * 4);
   w.row_off = (int64_t*)take(sizeof(int64_t) * (nb + 1));
   w.slot_off = (int64_t*)take(sizeof(int64_t) * (nb + 1));
   w.ell_rows = (int64_t*)take(sizeof(int64_t) * (nb > 0 ? nb : 1));
   w.totals = (int64_t*)take(sizeof(int64_t) * (ncat + 2));
-  w.err = (int32_t*)take(sizeof(int32_t) * 4);
   w.block_counts = (int32_t*)take(sizeof(int32_t) * blocks * ncat);
   w.block_offsets = (int64_t*)take(sizeof(int64_t) * blocks * ncat);
   w.bytes = off;
   return w;
 }
+
+// Host memory that ends with its scope (a C entry must not throw); p is null when there is none.
+struct HostBytes {
+  char* p;
+  explicit HostBytes(size_t n) : p((char*)calloc(n, 1)) {}
+  ~HostBytes() { free(p); }
+  HostBytes(const HostBytes&) = delete;
+  HostBytes& operator=(const HostBytes&) = delete;
+};
 
 int check_widths(int32_t num_parts, const int32_t* pbo, const int32_t* widths) {
   LF_REQUIRE(num_parts >= 1, "num_parts must be >= 1 (got %d)", num_parts);
@@ -781,10 +820,12 @@ int lf_hyb_stats(const int64_t* indptr, const int32_t* indices, int64_t num_rows
   unsigned int* long_count = (unsigned int*)long_base;
   LongSeg* long_list = (LongSeg*)(long_base + 256);
   const size_t n_stat = (size_t)num_parts * kClasses * 3;
-  LF_CUDA_CHECK(cudaMemsetAsync(colmask, 0, sizeof(uint32_t) * num_cols, st));
-  LF_CUDA_CHECK(cudaMemsetAsync(long_count, 0, sizeof(unsigned int), st));
-  LF_CUDA_CHECK(cudaMemsetAsync(class_stats, 0, sizeof(int64_t) * n_stat, st));
-  LF_CUDA_CHECK(cudaMemsetAsync(colmask_hist, 0, sizeof(int64_t) * (size_t)num_parts * LF_COLMASK_BINS, st));
+  const size_t n_hist = (size_t)num_parts * LF_COLMASK_BINS;
+  // the class masks with the counter behind them, and the two tables where they follow one another
+  LF_CUDA_CHECK(cudaMemsetAsync(colmask, 0, (size_t)(long_base - (char*)workspace) + sizeof(unsigned int), st));
+  const bool adjacent = class_stats + n_stat == colmask_hist;
+  LF_CUDA_CHECK(cudaMemsetAsync(class_stats, 0, sizeof(int64_t) * (n_stat + (adjacent ? n_hist : 0)), st));
+  if (!adjacent) LF_CUDA_CHECK(cudaMemsetAsync(colmask_hist, 0, sizeof(int64_t) * n_hist, st));
   if (num_rows > 0) {
     if (num_parts == 1) {
       const int64_t want = ceil_div64(num_rows, 8 * 32);  // 8 warps per block, 32 rows per warp and step
@@ -810,6 +851,13 @@ int lf_hyb_stats(const int64_t* indptr, const int32_t* indices, int64_t num_rows
     colmask_hist_kernel<<<grid, 256, 0, st>>>(colmask, num_cols, psz, (unsigned long long*)colmask_hist);
     LF_CUDA_CHECK(cudaGetLastError());
   }
+  return LF_OK;
+}
+
+int lf_hyb_class_coverage(int64_t* colmask_hist, int32_t num_parts, void* stream) {
+  LF_REQUIRE(colmask_hist && num_parts >= 1, "bad arguments");
+  class_coverage_kernel<<<(unsigned)num_parts, 512, 0, (cudaStream_t)stream>>>((unsigned long long*)colmask_hist);
+  LF_CUDA_CHECK(cudaGetLastError());
   return LF_OK;
 }
 
@@ -936,26 +984,28 @@ int lf_hyb_plan(const int64_t* indptr, const int32_t* indices, int64_t num_rows,
   const int64_t blocks = ceil_div64(rows > 0 ? rows : 1, kRowsPerBlock);
   LF_REQUIRE(blocks < (1ll << 31), "row range too large");
 
-  LF_CUDA_CHECK(cudaMemcpyAsync(ws.pbo, part_bucket_off, sizeof(int32_t) * (num_parts + 1), cudaMemcpyHostToDevice, st));
-  if (nb) LF_CUDA_CHECK(cudaMemcpyAsync(ws.widths, widths, sizeof(int32_t) * nb, cudaMemcpyHostToDevice, st));
-  LF_CUDA_CHECK(cudaMemsetAsync(ws.err, 0, sizeof(int32_t) * 4, st));
+  // one copy for the tables (they lie one behind the other; the error flag after them is 0), one read-back
+  // for the results: totals per category, the error flag and the end of the entry range (int32 guard).
+  // Four read-backs to pageable memory cost 15 us each.
+  char* dev = (char*)ws.pbo;
+  const size_t up_bytes = (size_t)((char*)ws.err - dev) + sizeof(int32_t) * 4;
+  HostBytes up(up_bytes), down(sizeof(int64_t) * (ncat + 2));
+  if (!up.p || !down.p) return fail(LF_ERR_CUDA, "lf_hyb_plan: out of host memory");
+  memcpy(up.p, part_bucket_off, sizeof(int32_t) * (num_parts + 1));
+  if (nb) memcpy(up.p + ((char*)ws.widths - dev), widths, sizeof(int32_t) * nb);
+  LF_CUDA_CHECK(cudaMemcpyAsync(dev, up.p, up_bytes, cudaMemcpyHostToDevice, st));
   hyb_count_kernel<<<(unsigned)blocks, kRowsPerBlock, sizeof(int32_t) * ncat, st>>>(
       indptr, indices, row_begin, row_end, (uint32_t)num_cols, psz, num_parts, ws.pbo, ws.widths, ncat,
       ws.block_counts, ws.err);
   LF_CUDA_CHECK(cudaGetLastError());
-  scan_blocks_kernel<<<ncat, 256, 0, st>>>(ws.block_counts, blocks, ncat, ws.block_offsets, ws.totals);
+  scan_blocks_kernel<<<ncat, 256, 0, st>>>(ws.block_counts, blocks, ncat, ws.block_offsets, ws.totals, ws.err,
+                                         indptr + row_end);
   LF_CUDA_CHECK(cudaGetLastError());
 
-  // host results: totals per category, the error flag and the entry range (for the int32 guard)
-  int64_t h_tot_small[64];
-  int64_t* h_tot = ncat <= 64 ? h_tot_small : (int64_t*)malloc(sizeof(int64_t) * ncat);
-  int32_t h_err = 0;
-  int64_t h_ptr[2] = {0, 0};
-  cudaError_t ce = cudaMemcpyAsync(h_tot, ws.totals, sizeof(int64_t) * ncat, cudaMemcpyDeviceToHost, st);
-  if (ce == cudaSuccess) ce = cudaMemcpyAsync(&h_err, ws.err, sizeof(int32_t), cudaMemcpyDeviceToHost, st);
-  if (ce == cudaSuccess) ce = cudaMemcpyAsync(&h_ptr[0], indptr + row_begin, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
-  if (ce == cudaSuccess) ce = cudaMemcpyAsync(&h_ptr[1], indptr + row_end, sizeof(int64_t), cudaMemcpyDeviceToHost, st);
+  const int64_t* h_tot = (const int64_t*)down.p;
+  cudaError_t ce = cudaMemcpyAsync(down.p, ws.totals, sizeof(int64_t) * (ncat + 2), cudaMemcpyDeviceToHost, st);
   if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+  const int32_t h_err = (int32_t)h_tot[ncat];
   int status = LF_OK;
   if (ce != cudaSuccess) {
     status = fail(LF_ERR_CUDA, "lf_hyb_plan: %s", cudaGetErrorString(ce));
@@ -963,7 +1013,7 @@ int lf_hyb_plan(const int64_t* indptr, const int32_t* indices, int64_t num_rows,
     status = fail(LF_ERR_INVALID_ARGUMENT, "the matrix holds a column index outside [0, %lld)", (long long)num_cols);
   } else if (h_err) {
     status = fail(LF_ERR_INVALID_ARGUMENT, "partition %d holds entries but was given no bucket width", h_err - 1);
-  } else if (h_ptr[1] > 0x7fffffffll) {
+  } else if (h_tot[ncat + 1] > 0x7fffffffll) {
     status = fail(LF_ERR_UNSUPPORTED, "more than 2^31-1 stored entries are not supported");
   } else {
     row_off[0] = slot_off[0] = 0;
@@ -974,7 +1024,6 @@ int lf_hyb_plan(const int64_t* indptr, const int32_t* indices, int64_t num_rows,
     }
     *num_zero_rows = h_tot[nb];
   }
-  if (h_tot != h_tot_small) free(h_tot);
   return status;
 }
 

@@ -46,9 +46,9 @@ def search_bucket_config(g: MTX, num_parts: int, cost_model_config: CostModelSet
     single nonzero, like the reference (format_algos.py:920-921).
     """
     csr = g.csr_device(device)
-    stats, hist = _hyb.hyb_stats(csr, int(num_parts))
-    return _ws.search_from_stats(stats, hist, int(cost_model_config.feat_size),
-                                 int(cost_model_config.num_parts))
+    stats, coverage = _hyb.hyb_coverage(csr, int(num_parts))
+    return _ws.search_from_coverage(stats, coverage, int(cost_model_config.feat_size),
+                                    int(cost_model_config.num_parts))
 
 
 def suggest_num_parts(g: MTX, feat_size: int, candidates=(1, 2, 4, 8, 16, 32), device="cuda"):
@@ -64,10 +64,10 @@ def suggest_num_parts(g: MTX, feat_size: int, candidates=(1, 2, 4, 8, 16, 32), d
     for P in candidates:
         if P > g.num_dst_nodes():
             continue
-        stats, hist = _hyb.hyb_stats(csr, int(P))
+        stats, coverage = _hyb.hyb_coverage(csr, int(P))
         per_part = []
         try:
-            _ws.search_from_stats(stats, hist, int(feat_size), int(P), cost_out=per_part)
+            _ws.search_from_coverage(stats, coverage, int(feat_size), int(P), cost_out=per_part)
         except ValueError:
             continue
         costs[int(P)] = float(sum(per_part))

@@ -98,6 +98,16 @@ class Workspace:
 
 def hyb_stats(csr: DeviceCsr, num_parts: int, workspace: Optional[Workspace] = None):
     """Run ``lf_hyb_stats``; returns ``(class_stats int64[P,11,3], colmask_hist int64[P,2048])`` on the host."""
+    return _stats(csr, num_parts, workspace, False)
+
+
+def hyb_coverage(csr: DeviceCsr, num_parts: int, workspace: Optional[Workspace] = None):
+    """``lf_hyb_stats`` + ``lf_hyb_class_coverage``: ``class_stats`` as ``hyb_stats`` and, instead of the
+    histogram, the columns touched by every set of classes, int64[P,2048]."""
+    return _stats(csr, num_parts, workspace, True)
+
+
+def _stats(csr, num_parts, workspace, coverage):
     torch = _torch()
     lib = _cabi.load()
     M, K = csr.shape
@@ -113,6 +123,8 @@ def hyb_stats(csr: DeviceCsr, num_parts: int, workspace: Optional[Workspace] = N
             ws = workspace.get(ws_bytes, 1)
         check(lib.lf_hyb_stats(t_ptr(csr.indptr), t_ptr(csr.indices), M, K, num_parts, out.data_ptr(),
                                out.data_ptr() + n_stat * 8, ws.data_ptr(), ws_bytes, _stream_ptr(torch)))
+        if coverage:
+            check(lib.lf_hyb_class_coverage(out.data_ptr() + n_stat * 8, num_parts, _stream_ptr(torch)))
         host = out.cpu().numpy()      # one read-back for both tables (synchronises the stream)
         return (host[:n_stat].reshape(num_parts, _cabi.NUM_WIDTH_CLASSES, 3).copy(),
                 host[n_stat:].reshape(num_parts, _cabi.COLMASK_BINS).copy())

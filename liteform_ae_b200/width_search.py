@@ -6,7 +6,7 @@ The reference keeps, per bucket, a Python list of row ids and a Python set of co
 lengths: three counters per (partition, width class) and, per partition, a 2048-bin
 histogram over the per-column bitmask of classes that touch the column.  A merged bucket is
 a set of classes; its number of distinct columns is the sum of the bins whose mask
-intersects that set.
+intersects that set, tabulated for every set at once (``coverage_from_hist``, or on the device).
 
 Everything order- or rounding-sensitive is kept as the reference has it:
   * a bucket that is created by a move lands at the END of the dict, and costs are summed
@@ -51,30 +51,24 @@ def _move(pool: Dict[int, _Bucket], src_w: int, dst_w: int) -> None:
     del pool[src_w]
 
 
-class _ColumnCounter:
-    """len(col_indices) of a merged bucket from the class-mask histogram of one partition."""
-
-    def __init__(self, hist_row: np.ndarray):
-        self._hist = np.asarray(hist_row, dtype=np.int64)
-        self._bins = np.arange(BINS, dtype=np.int64)
-        self._memo: Dict[int, int] = {}
-
-    def __call__(self, classes: int) -> int:
-        got = self._memo.get(classes)
-        if got is None:
-            got = int(self._hist[(self._bins & classes) != 0].sum())
-            self._memo[classes] = got
-        return got
+def coverage_from_hist(colmask_hist: np.ndarray) -> np.ndarray:
+    """int64[P, 2048] -> int64[P, 2048]: for every set of classes the columns that a class of the set
+    touches -- all of them less those whose mask lies inside the complement (``lf_hyb_class_coverage``)."""
+    f = np.array(colmask_hist, dtype=np.int64).reshape(-1, BINS)
+    for k in range(NUM_CLASSES):
+        pair = f.reshape(len(f), -1, 2, 1 << k)
+        pair[:, :, 1] += pair[:, :, 0]
+    return f[:, -1:] - f[:, ::-1]
 
 
-def _cost(pool: Dict[int, _Bucket], ncols: _ColumnCounter, feat_size: int, num_parts: int):
+def _cost(pool: Dict[int, _Bucket], ncols: np.ndarray, feat_size: int, num_parts: int):
     wmax = max(pool.keys())
     total = 0
     for w, b in pool.items():
         per_block = wmax // w
         padded = ((b.num_rows + per_block - 1) // per_block) * per_block
         c_index = 2 * padded * w
-        c_gather = ncols(b.classes) * feat_size
+        c_gather = int(ncols[b.classes]) * feat_size
         atomic = num_parts > 1 or w == wmax
         weight = padded / b.n_row_ids if atomic else 1
         c_out = weight * b.n_row_ids * feat_size
@@ -98,7 +92,7 @@ def _fix_single_row_buckets(pool: Dict[int, _Bucket]) -> None:
         _move(pool, 1, target)
 
 
-def _choose(pool: Dict[int, _Bucket], ncols: _ColumnCounter, feat_size: int, num_parts: int,
+def _choose(pool: Dict[int, _Bucket], ncols: np.ndarray, feat_size: int, num_parts: int,
             cost_out: list = None) -> List[int]:
     best_cost = _cost(pool, ncols, feat_size, num_parts)
     best = sorted(pool.keys())
@@ -119,8 +113,15 @@ def search_from_stats(class_stats: np.ndarray, colmask_hist: np.ndarray, feat_si
                       num_parts: int, cost_out: list = None) -> List[List[int]]:
     """``class_stats``: int64[P, 11, 3] = (num_rows, nnz, #rows); ``colmask_hist``: int64[P, 2048].
     ``cost_out`` (a list) receives the winning cost of every non-empty partition."""
+    hist = np.asarray(colmask_hist, dtype=np.int64).reshape(num_parts, BINS)
+    return search_from_coverage(class_stats, coverage_from_hist(hist), feat_size, num_parts, cost_out)
+
+
+def search_from_coverage(class_stats: np.ndarray, coverage: np.ndarray, feat_size: int,
+                         num_parts: int, cost_out: list = None) -> List[List[int]]:
+    """The same search on ``coverage[p, c]``, the columns of partition p that a class of the set c touches."""
     class_stats = np.asarray(class_stats, dtype=np.int64).reshape(num_parts, NUM_CLASSES, 3)
-    colmask_hist = np.asarray(colmask_hist, dtype=np.int64).reshape(num_parts, BINS)
+    coverage = np.asarray(coverage, dtype=np.int64).reshape(num_parts, BINS)
     pools: List[Dict[int, _Bucket]] = []
     for p in range(num_parts):
         pool: Dict[int, _Bucket] = {}
@@ -135,5 +136,5 @@ def search_from_stats(class_stats: np.ndarray, colmask_hist: np.ndarray, feat_si
         _fix_single_row_buckets(pool)
     out: List[List[int]] = []
     for p, pool in enumerate(pools):
-        out.append(_choose(pool, _ColumnCounter(colmask_hist[p]), feat_size, num_parts, cost_out) if pool else [])
+        out.append(_choose(pool, coverage[p], feat_size, num_parts, cost_out) if pool else [])
     return out
