@@ -84,8 +84,9 @@ const char* lf_last_error(void);
                                           copies, 2 or 4 = that many warps issuing per-lane cp.async */
 #define LF_OPT_BSR_BLOCK_WARPS 11       /* copy engine 1, more than 64 features: warps per thread block, 1..8 (0 = automatic:
                                           4 for 16-bit inputs up to 128 features, else 8) */
-#define LF_OPT_SPMM_RING_MIN_SLOTS 12    /* products with up to 64 float32 / 128 bf16 features: stored slots from which the
-                                          ring form (two launches) replaces the register kernel (default 2^20) */
+#define LF_OPT_SPMM_RING_MIN_SLOTS 12    /* stored slots from which a product whose B outgrows the L2 may take consecutive
+                                          slots per step, in two launches (default 2^20; 0: every product with
+                                          128-bit gathers does, whatever the size of B) */
 #define LF_OPT_SPMM_GATHER_RING 10      /* products with 128-bit gathers: where the gathered rows of B land: 16 (default) a
                                           ring of 16 rows (or steps of 2 / 4 narrow rows) per warp in shared memory,
                                           filled by cp.async; 0 registers (8 rows in flight per warp) */
@@ -237,7 +238,8 @@ int lf_spmm_hyb_f32(const lf_hyb* A, const float* B /*[dev] K x N*/, int64_t ldb
                     int32_t flags, void* stream);
 
 /* Name of the kernel lf_spmm_hyb_f32 launches for these operands under the current options
- * ("spmm_hyb_ring_kernel" or "spmm_hyb_kernel"); launches nothing.  For logs and benchmarks. */
+ * ("spmm_hyb_groups_kernel", "spmm_hyb_ring_rows_kernel", "spmm_hyb_ring_kernel" or "spmm_hyb_kernel"); launches
+ * nothing.  For logs and benchmarks. */
 const char* lf_spmm_hyb_f32_kernel_name(const lf_hyb* A, const float* B, int64_t ldb, const float* C, int64_t ldc,
                                         int32_t N);
 

@@ -201,7 +201,11 @@ int lf_spmm_csr_f32(const int64_t* indptr, const int32_t* indices, const float* 
   const FeatCfg cfg = pick_cfg(B, ldb, C, ldc, N);
   // the ring form multiplies row numbers by 32-bit pitches in bytes and keeps row numbers in 32 bits
   const bool ring = gather_ring() > 0 && ldb < (1ll << 30) && ldc < (1ll << 30) && row_end - row_begin < (1ll << 31) - 64;
-  const GroupCfg group = cfg.VEC == 4 ? pick_group(N, 4) : pick_group_shifted(N);
+  GroupCfg group = cfg.VEC == 4 ? pick_group(N, 4) : pick_group_shifted(N);
+  // one walk of full warps for up to 256 features (2^18 power-law rows at 200: 244 us, two walks of 128
+  // features 278); beyond that pieces of 128 (uniform rows, 300 features: two walks of 256 1543 us, three of
+  // 128 1239; 2^17 power-law rows at 384 217 / 200)
+  if (cfg.VEC == 4 && N > 128 && N <= 256) group = {32, 2, 1};
   const int gpc = kThreads / (ring ? group.G : cfg.G);
   // Entries per group.  Every range boundary cuts a row (cleared before, added to twice) and costs a
   // search, so long ranges win as soon as the grid fills the chip about twice; measured on

@@ -41,13 +41,12 @@ template <int G> constexpr int kGroupStrips = G == 4 ? 4 : 2;   // strips held: 
 // Lanes per group, chunks per lane and the number of walks (blocks along y) for N features.
 struct GroupCfg { int G, CH, passes; };
 // 16-byte aligned rows of `vec` features per chunk: groups as narrow as the row, two chunks per
-// lane for rows of more than 128 bytes.
+// lane for rows of more than 128 bytes, pieces of 512 bytes for wider ones.
 inline GroupCfg pick_group(int N, int vec) {
   if (N <= 4 * vec) return {4, 1, 1};
   if (N <= 8 * vec) return {8, 1, 1};
   if (N <= 16 * vec) return {8, 2, 1};
-  if (N <= 32 * vec) return {16, 2, 1};
-  return {32, 2, (N + 64 * vec - 1) / (64 * vec)};
+  return {16, 2, (N + 32 * vec - 1) / (32 * vec)};
 }
 // Shifted rows: a group of G lanes takes 4 G - 4 features behind any shift; a third of a full warp's
 // time per walk is work that fewer lanes do not save.

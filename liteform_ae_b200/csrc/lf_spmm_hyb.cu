@@ -24,12 +24,12 @@
 //     0 * Inf and 0 * NaN from B do not reach C (SciPy would produce NaN there);
 //   * by default the products with 128-bit gathers run a second form of the same walk whose gathers
 //     land in a per-lane shared-memory ring (cp.async, 16 rows ahead) instead of registers: see
-//     spmm_hyb_ring_kernel (rows of B that fill a warp) and spmm_hyb_ring_rows_kernel (rows of 8
-//     or 16 lanes, several slots per step);
+//     spmm_hyb_ring_kernel (rows of B that fill a warp), spmm_hyb_ring_rows_kernel (rows or pieces of 8
+//     or 16 lanes, several slots per step) and, while B stays in the L2, spmm_hyb_groups_kernel;
 //   * variants of the same code: B in bf16 (8 features per lane), and a broadcasting epilogue that
 //     stores every row into several full-size C matrices (the GPUs of a group) at once.
 #include "lf_bsr8_tma.cuh"
-#include "lf_spmm_gather.cuh"
+#include "lf_spmm_group.cuh"
 
 namespace lf {
 
@@ -82,6 +82,25 @@ struct SpmmTable {
   int32_t seg_tiles;      // thread blocks per segment over all buckets (0 = bucket-major)
   BucketDesc b[MAXB];
 };
+
+// The bucket of the calling thread block and the block's position inside it.
+template <int MAXB>
+__device__ __forceinline__ const BucketDesc& bucket_of_block(const SpmmTable<MAXB>& tbl, int64_t& tile) {
+  int64_t key = blockIdx.x;
+  uint32_t seg = 0;
+  if (tbl.seg_tiles > 0) {
+    seg = (uint32_t)blockIdx.x / (uint32_t)tbl.seg_tiles;
+    key = (uint32_t)blockIdx.x - seg * (uint32_t)tbl.seg_tiles;
+  }
+  int lo = 0, hi = tbl.n;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (tbl.b[mid].tile_begin <= key) lo = mid; else hi = mid;
+  }
+  const BucketDesc& d = tbl.b[lo];
+  tile = tbl.seg_tiles > 0 ? (int64_t)seg * d.tiles_per_seg + (key - d.tile_begin) : key - d.tile_begin;
+  return d;
+}
 
 // One thread group walks the slots [s0, s1) of whole ELL rows of one bucket.
 //   G lanes per group, V chunks of VEC floats per lane: one pass covers G*V*VEC features.
@@ -202,20 +221,8 @@ spmm_hyb_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int32_t* __re
   __shared__ int2 s_cv[kThreads];
   __shared__ int s_rd[kThreads];
 
-  int64_t tile = blockIdx.x;   // position of this thread block inside its bucket, once found
-  int64_t key = tile;
-  uint32_t seg = 0;
-  if (tbl.seg_tiles > 0) {
-    seg = (uint32_t)blockIdx.x / (uint32_t)tbl.seg_tiles;
-    key = (uint32_t)blockIdx.x - seg * (uint32_t)tbl.seg_tiles;
-  }
-  int lo = 0, hi = tbl.n;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (tbl.b[mid].tile_begin <= key) lo = mid; else hi = mid;
-  }
-  const BucketDesc& d = tbl.b[lo];
-  tile = tbl.seg_tiles > 0 ? (int64_t)seg * d.tiles_per_seg + (key - d.tile_begin) : key - d.tile_begin;
+  int64_t tile;
+  const BucketDesc& d = bucket_of_block(tbl, tile);
   const int wlog = d.wlog;
   const int g = threadIdx.x / G, lane = threadIdx.x % G;
   const unsigned gmask = G == 32 ? 0xffffffffu : (((1u << G) - 1u) << ((threadIdx.x & 31) / G * G));
@@ -412,20 +419,8 @@ spmm_hyb_ring_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int32_t*
   __shared__ __align__(16) float s_val[GPC * 64];
   __shared__ int s_rd[GPC * 64];
 
-  int64_t tile = blockIdx.x;
-  int64_t key = tile;
-  uint32_t seg = 0;
-  if (tbl.seg_tiles > 0) {
-    seg = (uint32_t)blockIdx.x / (uint32_t)tbl.seg_tiles;
-    key = (uint32_t)blockIdx.x - seg * (uint32_t)tbl.seg_tiles;
-  }
-  int lo = 0, hi = tbl.n;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (tbl.b[mid].tile_begin <= key) lo = mid; else hi = mid;
-  }
-  const BucketDesc& d = tbl.b[lo];
-  tile = tbl.seg_tiles > 0 ? (int64_t)seg * d.tiles_per_seg + (key - d.tile_begin) : key - d.tile_begin;
+  int64_t tile;
+  const BucketDesc& d = bucket_of_block(tbl, tile);
   const int wlog = d.wlog;
   const int g = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t e0 = (tile * GPC + g) * (int64_t)d.rows_per_group;
@@ -614,20 +609,8 @@ spmm_hyb_ring_rows_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int
   __shared__ __align__(16) float s_val[GPC * NB * 32];
   __shared__ int s_rd[GPC * NB * 32];
 
-  int64_t tile = blockIdx.x;
-  int64_t key = tile;
-  uint32_t seg = 0;
-  if (tbl.seg_tiles > 0) {
-    seg = (uint32_t)blockIdx.x / (uint32_t)tbl.seg_tiles;
-    key = (uint32_t)blockIdx.x - seg * (uint32_t)tbl.seg_tiles;
-  }
-  int lo = 0, hi = tbl.n;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (tbl.b[mid].tile_begin <= key) lo = mid; else hi = mid;
-  }
-  const BucketDesc& d = tbl.b[lo];
-  tile = tbl.seg_tiles > 0 ? (int64_t)seg * d.tiles_per_seg + (key - d.tile_begin) : key - d.tile_begin;
+  int64_t tile;
+  const BucketDesc& d = bucket_of_block(tbl, tile);
   const int wlog = d.wlog;
   const int g = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t e0 = (tile * GPC + g) * (int64_t)d.rows_per_group;
@@ -648,6 +631,39 @@ spmm_hyb_ring_rows_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int
     case 2: LF_WALK(4); break;
     default: LF_WALK(8); break;
   }
+#undef LF_WALK
+}
+
+// ---- a row of B per group of lanes ----------------------------------------------------------------
+// The form for a B that stays in the L2, where instructions per row bound the time: every group of
+// lanes, as narrow as a row of B, walks ELL rows of its own through the group ring (lf_spmm_group.cuh),
+// one launch for buckets of any width.  Rows are added up in the order of the register kernel.
+template <int G, int CH, int VEC, int MAXB>
+__global__ void __launch_bounds__(kThreads, CH == 1 ? 4 : 3)
+spmm_hyb_groups_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int32_t* __restrict__ rows_arena,
+                       const int32_t* __restrict__ cols_arena, const float* __restrict__ vals_arena,
+                       const typename BTraits<VEC>::elem* __restrict__ B, int ldb, float* __restrict__ C, int64_t ldc,
+                       int N, int64_t row_base) {
+  extern __shared__ __align__(16) unsigned char ring_bytes[];
+  constexpr int R = 32 / G, GPC = kThreads / G, kFeatures = kGroupFeatures<G, CH, VEC, false>;
+  int64_t tile;
+  const BucketDesc& d = bucket_of_block(tbl, tile);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane / G, gl = lane % G;
+  const int64_t first = (tile * GPC + w * R) * (int64_t)d.rows_per_group;   // the warp's first ELL row
+  if (first >= d.ell_rows) return;
+  const int64_t e0 = min(first + g * (int64_t)d.rows_per_group, d.ell_rows), e1 = min(e0 + d.rows_per_group, d.ell_rows);
+  const int wlog = d.wlog;
+  const int64_t at = d.slot_off + (e0 << wlog);
+  EllRowIds<G> ids;
+  ids.init(rows_arena + d.row_off, wlog, e0, e1, d.ell_rows);
+  const int f0 = blockIdx.y * kFeatures;
+#define LF_WALK(WC_)                                                                                            \
+  walk_group_ring<G, CH, VEC, false, WC_>(ids, d.force_atomic != 0, cols_arena + at, vals_arena + at, B + f0, ldb, \
+                                          C - row_base * ldc + f0, ldc, min(N - f0, kFeatures), g, gl,          \
+                                          ring_bytes + w * GroupSmem<G, CH, false>::kBytes)
+  if (wlog == 0) LF_WALK(1);
+  else if (wlog == 1) LF_WALK(2);
+  else LF_WALK(4);
 #undef LF_WALK
 }
 
@@ -721,7 +737,7 @@ FeatCfg pick_cfg_bf16(int N) {
 }
 
 // Process-wide tuning knobs (lf_set_option); the environment gives the initial values.
-// stored slots from which rows of B narrower than a warp take the two-launch ring path (LF_OPT_SPMM_RING_MIN_SLOTS)
+// stored slots from which a product may take the two launches of consecutive slots per step (LF_OPT_SPMM_RING_MIN_SLOTS)
 int g_ring_rows_min_slots = 1 << 20;
 int g_slots_per_group = 0;
 int g_cache_policy = -1;
@@ -838,9 +854,39 @@ int launch_hyb_ring_rows(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb
 #undef LF_ROWS
 }
 
+// A row of B per group of lanes.
+template <int MAXB, int VEC>
+int launch_hyb_groups(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, const void* B, int64_t ldb, float* C,
+                      int64_t ldc, int N, GroupCfg group, cudaStream_t st, bool dep) {
+  const dim3 grid((unsigned)tiles, (unsigned)group.passes);
+#define LF_GROUPS(G_, CH_)                                                                                      \
+  do {                                                                                                          \
+    constexpr auto kern = spmm_hyb_groups_kernel<G_, CH_, VEC, MAXB>;                                           \
+    constexpr int smem = kThreads / 32 * GroupSmem<G_, CH_, false>::kBytes;                                     \
+    LF_CUDA_CHECK(allow_smem<kern>(smem));                                                                      \
+    LF_CUDA_CHECK(launch_dep_smem(kern, grid, kThreads, smem, st, dep, tbl, A->rows, A->cols, A->vals,          \
+                                  (const typename BTraits<VEC>::elem*)B, (int)ldb, C, ldc, N, A->row_begin));   \
+    return LF_OK;                                                                                               \
+  } while (0)
+  if (group.G == 4) LF_GROUPS(4, 1);
+  else if (group.G == 8 && group.CH == 1) LF_GROUPS(8, 1);
+  else if (group.G == 8) LF_GROUPS(8, 2);
+  else LF_GROUPS(16, 2);
+#undef LF_GROUPS
+}
+
+// Which kernel takes a product: rows of B by groups of lanes, several consecutive slots per step (and
+// the buckets narrower than those in a launch of their own), or the rest (launch_hyb: a ring per warp,
+// registers).
+enum class Form { kGroups, kSlots, kOther };
+
 template <int MAXB>
 int launch_hyb(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, const void* Bv, int64_t ldb,
-               float* C, int64_t ldc, int N, FeatCfg cfg, cudaStream_t st, const DestList& dests, bool dep) {
+               float* C, int64_t ldc, int N, FeatCfg cfg, Form form, GroupCfg group, cudaStream_t st,
+               const DestList& dests, bool dep) {
+  if (form == Form::kGroups && cfg.VEC == 8) return launch_hyb_groups<MAXB, 8>(tbl, tiles, A, Bv, ldb, C, ldc, N, group, st, dep);
+  if (form == Form::kGroups) return launch_hyb_groups<MAXB, 4>(tbl, tiles, A, Bv, ldb, C, ldc, N, group, st, dep);
+  if (form == Form::kSlots) return launch_hyb_ring_rows<MAXB>(tbl, tiles, A, Bv, cfg.VEC == 8, ldb, C, ldc, N, cfg.G, st, dep);
   if (cfg.VEC == 8)   // bf16 B: one compiled variant per feature layout
     return launch_hyb_bf16<MAXB>(tbl, tiles, A, (const uint16_t*)Bv, ldb, C, ldc, N, cfg, st, dests, dep);
   const float* B = (const float*)Bv;
@@ -870,6 +916,33 @@ int launch_hyb(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, const
   LF_CASE(1, 2); LF_CASE(1, 3); LF_CASE(1, 4);
 #undef LF_CASE
   return fail(LF_ERR_INVALID_ARGUMENT, "bad tuning state");
+}
+
+// The rule.  All of it is for 16-byte gathers and 32-bit pitches in bytes; operands off that grid stay with
+// the registers (473 062 power-law rows, 27 features, 4 partitions: 161 us, shifted copies into a ring 212 us).
+// "Touched" is what the stored slots can reach of B; times are us, form on the other side / form taken.
+//   * By groups while that stays in the L2 beside what streams through.  2^18 power-law rows: 32 features
+//     (34 MB) 65 / 47, 64 (67 MB) 81 / 76 and with 4 partitions 121 / 103; 100 000 Zipf rows at 200 features,
+//     2 partitions (80 MB) 154 / 135; 4000 at 512 29 / 18.  Past it: 400 000 uniform rows at 64 features
+//     (102 MB) groups 244, consecutive slots 225; 2^18 power-law rows at 100 features (105 MB) 173, ring per warp 164.
+//     Rows of up to 128 bytes, where the other form has four partial sums to add, a little longer: 2^20
+//     power-law rows at 24 features, 8 partitions (101 MB) 311 / 250; at 134 MB of uniform rows 424 against 457.
+//     bf16 rows of more than 256 bytes keep the ring per warp (16 234 Zipf rows, 240 features: 27.4, groups 28.7).
+//   * bf16 rows of more than 256 bytes in pieces of 256 bytes, by consecutive slots, once 512-byte pieces of
+//     B are more than twice the L2: a piece finds more of itself there.  256 features: 2^20 skewed rows 1748 /
+//     1682, uniform 2318 / 1998, 2^19 power-law rows with 8 partitions 1091 / 1003.  In float32 a uniform matrix
+//     gains as much (2^20 rows at 128 features 2236 / 1915) but the power-law graph gains nothing (564 to 571
+//     either way, 648 / 665 on another card) and loses to the second reading of the slots below that size
+//     (2^18 rows at 256 features 236 / 279): float32 keeps the ring per warp.
+Form form_of(const lf_hyb* A, const FeatCfg& cfg, int64_t ldb, int64_t ldc, int N, bool several_dests) {
+  if (gather_ring() == 0 || cache_policy() != 1 || cfg.VEC == 1 || several_dests || ldb >= (1ll << 30)) return Form::kOther;
+  const int64_t slots = A->slot_off[A->num_buckets], reach = A->num_cols < slots ? A->num_cols : slots;
+  const int64_t row = (int64_t)N * (cfg.VEC == 8 ? 2 : 4);
+  const int64_t resident = (row <= 128 ? 104ll : 80ll) << 20;
+  if (g_ring_rows_min_slots > 0 && reach * row <= resident && ldc < (1ll << 30) && (row <= 256 || cfg.VEC == 4)) return Form::kGroups;
+  if (slots < g_ring_rows_min_slots) return Form::kOther;
+  const bool pieces = (cfg.VEC == 8 && reach * 512 >= (256ll << 20)) || g_ring_rows_min_slots == 0;
+  return row <= 256 || pieces ? Form::kSlots : Form::kOther;
 }
 
 int check_hyb(const lf_hyb* A) {
@@ -964,9 +1037,11 @@ const char* lf_spmm_hyb_f32_kernel_name(const lf_hyb* A, const float* B, int64_t
                                         int32_t N) {
   if (!A || N < 1) return "";
   const FeatCfg cfg = pick_cfg(B, ldb, C, ldc, N);
-  if (gather_ring() > 0 && cfg.VEC == 4 && cfg.G < 32 && ldb < (1ll << 30) && cache_policy() == 1 &&
-      A->slot_off && A->slot_off[A->num_buckets] >= g_ring_rows_min_slots)
-    return "spmm_hyb_ring_rows_kernel";   // buckets narrower than 32 / lanes-per-row slots: spmm_hyb_kernel
+  switch (A->slot_off ? form_of(A, cfg, ldb, ldc, N, false) : Form::kOther) {
+    case Form::kGroups: return "spmm_hyb_groups_kernel";
+    case Form::kSlots: return "spmm_hyb_ring_rows_kernel";   // buckets narrower than the slots of a step: spmm_hyb_kernel
+    default: break;
+  }
   return gather_ring() > 0 && ring_applies(cfg, ldb) ? "spmm_hyb_ring_kernel" : "spmm_hyb_kernel";
 }
 
@@ -1007,7 +1082,7 @@ static int spmm_hyb_impl(const lf_hyb* A, const void* B, bool b_is_bf16, int64_t
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t shard_rows = A->row_end - A->row_begin;
   if (shard_rows == 0) return LF_OK;
-  const FeatCfg cfg = b_is_bf16 ? pick_cfg_bf16(N) : pick_cfg(B, ldb, C, ldc, N);
+  FeatCfg cfg = b_is_bf16 ? pick_cfg_bf16(N) : pick_cfg(B, ldb, C, ldc, N);
   const bool accumulate = flags == LF_SPMM_ACCUMULATE;
   const bool all_atomic = accumulate || A->num_parts > 1;
   bool cleared_by_kernel = false;   // a row-clearing launch precedes: the product depends on it programmatically
@@ -1041,27 +1116,26 @@ static int spmm_hyb_impl(const lf_hyb* A, const void* B, bool b_is_bf16, int64_t
     }
   }
 
-  // Rows of B narrower than a warp (8 or 16 lanes): buckets at least as wide as the slots of a step
-  // go to the ring kernel that takes several slots per step, the narrower ones to the register
-  // kernel in a launch of their own.
-  // Small products stay with the one launch of the register kernel (a 16384-row matrix: 0.013 ms
-  // against 0.023 ms for the two launches).
+  const Form form = form_of(A, cfg, ldb, ldc, N, dests.n > 0);
+  GroupCfg group = {0, 0, 1};
+  if (form == Form::kGroups) group = pick_group(N, cfg.VEC);
+  if (form == Form::kSlots && cfg.G == 32) cfg = {16, 1, cfg.VEC, 16 * cfg.VEC};   // pieces of 256 bytes
   const int rows_per_step = 32 / cfg.G;
-  const bool split = gather_ring() > 0 && cfg.VEC != 1 && rows_per_step > 1 && dests.n == 0 && ldb < (1ll << 30) &&
-                     cache_policy() == 1 && A->slot_off[A->num_buckets] >= g_ring_rows_min_slots;
   const int segs = tile_segments();
-  for (int pass = 0; pass < (split ? 2 : 1); ++pass) {
-    const bool ring_rows = split && pass == 0;
+  for (int pass = 0; pass < (form == Form::kSlots ? 2 : 1); ++pass) {
+    const Form f = pass == 0 ? form : Form::kOther;
     // one launch per LF_MAX_BUCKETS_PER_LAUNCH non-empty buckets (one launch in every practical case)
-    const int gpc = ring_rows ? kThreads / 32 : kThreads / cfg.G;
+    const int gpc = f == Form::kSlots ? kThreads / 32 : kThreads / (f == Form::kGroups ? group.G : cfg.G);
     auto in_pass = [&](int k) {
       if (A->ell_rows[k] == 0) return false;
-      if (!split) return true;
-      return (A->widths[k] >= rows_per_step) == ring_rows;
+      return form != Form::kSlots || (A->widths[k] >= rows_per_step) == (pass == 0);
     };
+    // A block of the group form takes up to 16384 slots: four waves of blocks are enough (2^18 power-law
+    // rows, 64 features, 4 partitions: 1 / 2 / 4 / 8 waves 160 / 112 / 101 / 100 us), and longer runs pay where
+    // a row of 100 000 entries is added up by all of them.
     int spg = slots_per_group();
     if (!spg) {
-      const int64_t want_tiles = (int64_t)sm_count() * min_blocks() * 8;
+      const int64_t want_tiles = (int64_t)sm_count() * min_blocks() * (f == Form::kGroups ? 4 : 8);
       for (spg = 256; spg > 32; spg >>= 1) {
         int64_t t = 0;
         for (int k = 0; k < A->num_buckets; ++k) {
@@ -1070,7 +1144,7 @@ static int spmm_hyb_impl(const lf_hyb* A, const void* B, bool b_is_bf16, int64_t
           const int rpg = spg / w > 0 ? spg / w : 1;
           t += ceil_div64(A->ell_rows[k], (int64_t)rpg * gpc);
         }
-        if (t >= want_tiles) break;
+        if (t * group.passes >= want_tiles) break;
       }
     }
     int i = 0;
@@ -1107,13 +1181,11 @@ static int spmm_hyb_impl(const lf_hyb* A, const void* B, bool b_is_bf16, int64_t
         small.n = n;
         small.seg_tiles = (int32_t)(segs > 0 ? seg_tiles : 0);
         for (int k = 0; k < n; ++k) small.b[k] = big.b[k];
-        s = ring_rows ? launch_hyb_ring_rows<16>(small, grid_tiles, A, B, b_is_bf16, ldb, C, ldc, N, cfg.G, st, cleared_by_kernel)
-                      : launch_hyb<16>(small, grid_tiles, A, B, ldb, C, ldc, N, cfg, st, dests, cleared_by_kernel);
+        s = launch_hyb<16>(small, grid_tiles, A, B, ldb, C, ldc, N, cfg, f, group, st, dests, cleared_by_kernel);
       } else {
         big.n = n;
         big.seg_tiles = (int32_t)(segs > 0 ? seg_tiles : 0);
-        s = ring_rows ? launch_hyb_ring_rows<LF_MAX_BUCKETS_PER_LAUNCH>(big, grid_tiles, A, B, b_is_bf16, ldb, C, ldc, N, cfg.G, st, cleared_by_kernel)
-                      : launch_hyb<LF_MAX_BUCKETS_PER_LAUNCH>(big, grid_tiles, A, B, ldb, C, ldc, N, cfg, st, dests, cleared_by_kernel);
+        s = launch_hyb<LF_MAX_BUCKETS_PER_LAUNCH>(big, grid_tiles, A, B, ldb, C, ldc, N, cfg, f, group, st, dests, cleared_by_kernel);
       }
       if (s) return s;
       cleared_by_kernel = false;   // a further launch follows a product kernel, not the clearing one
