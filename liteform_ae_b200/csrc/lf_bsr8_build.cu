@@ -23,16 +23,9 @@ namespace {
 
 constexpr int kBuildThreads = 64;
 constexpr int kRowsPerCta = kBuildThreads / 8;   // block rows per thread block
-constexpr int kWindow = 32;                      // entries held of a row when the warp's rows do not fit
-constexpr int kStage = 2048;                     // entries a warp holds in shared memory
-// entry e of a warp's stage lies at e + e / 32: rows of 32, 64, ... entries do not share one bank
-__device__ __forceinline__ int staged(int e) { return e + (e >> 5); }
-constexpr int kStageWords = kStage + kStage / 32;
 constexpr int kNoBlock = 0x7fffffff;
 
-__device__ __forceinline__ void cp_async_4(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
-}
+__device__ __forceinline__ bool on_16_bytes(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 __device__ __forceinline__ int group_min8(int v) {
   v = min(v, __shfl_xor_sync(0xffffffffu, v, 1));
   v = min(v, __shfl_xor_sync(0xffffffffu, v, 2));
@@ -51,159 +44,141 @@ __device__ __forceinline__ uint32_t bits(__half x) { return __half_as_ushort(x);
 // FILL = false: counts[I + 1] = number of blocks of block row I.
 // FILL = true: writes block columns and tiles at bsr_indptr[I] + k for the k-th block.
 //
-// What bounds it: the entries' way from memory (a step of the merge is a handful of shared-memory reads).
-// A lane that walks its row in global memory has one 4-byte load in flight and waits for each.  Here a
-// warp copies the entries of its 32 rows, one contiguous range, into shared memory in one go where they
-// fit; otherwise it holds a window of 32 entries of each row and refills the windows that run low
-// together, eight rows in flight.  A step reads the up to eight entries of the block at once, and a full
-// tile row takes them in order.  2^18 rows of 64 entries in 8x8 blocks to fp16 tiles, the whole call (count,
-// scan, fill, two waits of the host): a load at a time 325 us, windows alone 178 us, this 139 us.
+// What bounds it: the chain of one step, from the columns a lane has next through the minimum over the
+// group to the columns after those; the longest block row of the matrix walks it once per block.  A lane
+// keeps the columns of its next eight entries in registers, so that the chain holds no load where blocks
+// are scattered (one entry of a row per block: the window moves up by one, the load at its end is needed
+// eight entries later), and two 16-byte loads where they are full (eight entries of a row per block).
+// Whole call (count, scan, fill, two waits of the host), 2^18 rows to fp16 tiles: an entry at a time from memory
+// / rows staged in shared memory / this, us: 8 full blocks per row 323 / 141 / 135, 9 291 / 246 / 123, 16
+// 557 / 366 / 229; 32 uniform columns per row 1185 / 1874 / 762, Zipf rows of up to 2048 entries
+// 3557 / 7730 / 2607, power-law rows of up to 50 000 17 098 / 29 958 / 13 720.
 template <bool FILL, typename T>
 __global__ void __launch_bounds__(kBuildThreads)
 bsr8_walk_kernel(const int64_t* __restrict__ indptr, const int32_t* __restrict__ indices,
                  const float* __restrict__ data, int64_t M, int64_t Mb, int64_t* __restrict__ bsr_indptr,
                  int32_t* __restrict__ bsr_indices, T* __restrict__ blocks) {
-  __shared__ int32_t s_col[kBuildThreads / 32 * kStageWords];
-  __shared__ float s_val[FILL ? kBuildThreads / 32 * kStageWords : 1];
-  const int l = threadIdx.x & 7, lane = threadIdx.x & 31;
+  const int l = threadIdx.x & 7;
   // whole warps stay in the loop together (the shuffles name all 32 lanes): block rows past Mb
   // simply have nothing to merge
   const int64_t I = (int64_t)blockIdx.x * kRowsPerCta + (threadIdx.x >> 3);
   const int64_t row = I * 8 + l;
   const bool live = I < Mb && row < M;
-  int64_t pos = live ? indptr[row] : 0;
-  const int64_t end = live ? indptr[row + 1] : 0;
+  const int64_t pos = live ? indptr[row] : 0, entries = live ? indptr[row + 1] - pos : 0;
   int64_t out = (FILL && I < Mb) ? bsr_indptr[I] : 0;
   int count = 0;
-  int32_t* col_stage = s_col + (threadIdx.x >> 5) * kStageWords;
-  float* val_stage = s_val + (FILL ? (threadIdx.x >> 5) * kStageWords : 0);
-  int last = kNoBlock;                  // block of the step before
-  int have = 0, off = lane * kWindow;   // entries pos .. pos + have - 1 lie at off in the stage
-  {
-    const int64_t from = __shfl_sync(0xffffffffu, pos, 0);   // the warp's first row is live if any is
-    int64_t to = end;
+  const int32_t* ip = indices + pos;                 // the row's next entry
+  const float* vp = data ? data + pos : nullptr;
+  int rem = entries > 0x7fffffff ? 0x7fffffff : (int)entries;   // entries from there on
+  int c[8];                                          // columns of the first eight of them
+  auto load_window = [&]() {
 #pragma unroll
-    for (int o = 16; o; o >>= 1) {
-      const int64_t x = __shfl_xor_sync(0xffffffffu, to, o);
-      to = x > to ? x : to;
-    }
-    if (__all_sync(0xffffffffu, !live || (from <= pos && pos <= end)) && to - from <= kStage) {
-      const int total = (int)(to - from);
-      const uint32_t col_s = (uint32_t)__cvta_generic_to_shared(col_stage), val_s = (uint32_t)__cvta_generic_to_shared(val_stage);
-#pragma unroll 4
-      for (int e = lane; e < total; e += 32) {
-        cp_async_4(col_s + staged(e) * 4, indices + from + e);
-        if (FILL && data) cp_async_4(val_s + staged(e) * 4, data + from + e);
-        if (FILL && !data) val_stage[staged(e)] = 1.0f;
-      }
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncwarp();
-      if (live) {
-        off = (int)(pos - from);
-        have = (int)(end - pos);
-      }
-    }
-  }
+    for (int k = 0; k < 8; ++k) c[k] = k < rem ? ip[k] : 0;
+  };
+  auto load_window_16 = [&]() {   // eight entries or more, on a 16-byte boundary
+    const int4 a = __ldg(reinterpret_cast<const int4*>(ip)), b = __ldg(reinterpret_cast<const int4*>(ip) + 1);
+    c[0] = a.x; c[1] = a.y; c[2] = a.z; c[3] = a.w;
+    c[4] = b.x; c[5] = b.y; c[6] = b.z; c[7] = b.w;
+  };
+  if (__all_sync(0xffffffffu, rem >= 8 && on_16_bytes(ip))) load_window_16();
+  else load_window();
   for (;;) {
-    // windows with less than a block's eight entries, though the row has more, are loaded again from pos
-    const bool low = have < 8 && pos + have < end;
-    unsigned todo = __ballot_sync(0xffffffffu, low);
-    if (todo) {
-      __syncwarp();
-      const int fresh = low ? (int)(end - pos < kWindow ? end - pos : kWindow) : 0;
-      while (todo) {
-        int at[8];
-        int32_t c[8];
-        float v[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int src = todo ? __ffs(todo) - 1 : 0;
-          const int64_t from = __shfl_sync(0xffffffffu, pos, src);
-          const int n = __shfl_sync(0xffffffffu, fresh, src);
-          const bool in = todo && lane < n;
-          at[u] = in ? staged(src * kWindow + lane) : -1;
-          c[u] = in ? indices[from + lane] : 0;
-          if (FILL) v[u] = in && data ? data[from + lane] : 1.0f;
-          todo &= todo - 1;   // 0 stays 0
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          if (at[u] >= 0) {
-            col_stage[at[u]] = c[u];
-            if (FILL) val_stage[at[u]] = v[u];
-          }
-        }
-      }
-      if (low) {
-        have = fresh;
-        off = lane * kWindow;
-      }
-      __syncwarp();
-    }
-    const int mine = have > 0 ? (col_stage[staged(off)] >> 3) : kNoBlock;
-    // only a row with repeated columns has entries of the last block left: they go into its tile one by one
-    const bool left = have > 0 && mine == last;
-    if (__any_sync(0xffffffffu, left)) {
-      if (left) {
-        int used = 0;
-        for (; pos < end && (indices[pos] >> 3) == last; ++pos, ++used)
-          if (FILL) blocks[(out - 1) * 64 + l * 8 + (indices[pos] & 7)] = from_float<T>(data ? data[pos] : 1.0f);
-        off += used;
-        have = have > used ? have - used : 0;
-      }
-      continue;
-    }
+    const int mine = rem > 0 ? c[0] >> 3 : kNoBlock;
     const int J = group_min8(mine);
     if (__all_sync(0xffffffffu, J == kNoBlock)) break;
-    if (J == kNoBlock) continue;   // this group is done, another group of the warp is not
-    // the row's entries inside block J: the first n of the stage
-    int col[8], n = 0;
-    bool run = true, dense = true;   // dense: all eight columns of the block, in order
+    // (a group that is done goes along, without entries, while another group of the warp is not)
+    const bool one = rem > 0 && mine == J;
+    T tile_row[8];
+    if (FILL) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      col[k] = k < have ? col_stage[staged(off + k)] : 0;
-      run = run && k < have && (col[k] >> 3) == J;
-      n += run ? 1 : 0;
-      dense = dense && run && (col[k] & 7) == k;
+      for (int k = 0; k < 8; ++k) tile_row[k] = from_float<T>(0.f);
+    }
+    bool left = false;   // only a row with repeated columns has entries of the block left
+    if (!__any_sync(0xffffffffu, one && rem > 1 && (c[1] >> 3) == J)) {   // scattered blocks
+      if (one) {
+        if (FILL) {
+          const T v = from_float<T>(vp ? *vp++ : 1.0f);
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if ((c[0] & 7) == k) tile_row[k] = v;
+        }
+#pragma unroll
+        for (int k = 0; k < 7; ++k) c[k] = c[k + 1];
+        if (rem > 8) c[7] = ip[8];
+        ++ip;
+        --rem;
+      }
+    } else {
+      int n = 0;                       // the row's entries inside block J: the first n
+      bool run = one, full = true;     // full: all eight columns of the block, in order
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        run = run && k < rem && (c[k] >> 3) == J;
+        n += run ? 1 : 0;
+        full = full && run && (c[k] & 7) == k;
+      }
+      const bool whole = full && on_16_bytes(ip) && (!FILL || !vp || on_16_bytes(vp)) && (rem == 8 || rem >= 16);
+      if (__all_sync(0xffffffffu, n == 0 || whole)) {
+        if (n) {
+          if (FILL) {
+            float4 a = make_float4(1.f, 1.f, 1.f, 1.f), b = a;
+            if (vp) {
+              a = __ldg(reinterpret_cast<const float4*>(vp));
+              b = __ldg(reinterpret_cast<const float4*>(vp) + 1);
+              vp += 8;
+            }
+            const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) tile_row[k] = from_float<T>(v[k]);
+          }
+          ip += 8;
+          rem -= 8;
+          if (rem) load_window_16();
+        }
+      } else if (n) {
+        if (FILL) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            if (k < n) {
+              const T v = from_float<T>(vp ? vp[k] : 1.0f);
+#pragma unroll
+              for (int j = 0; j < 8; ++j)
+                if ((c[k] & 7) == j) tile_row[j] = v;
+            }
+          }
+          if (vp) vp += n;
+        }
+        ip += n;
+        rem -= n;
+        load_window();
+        left = n == 8 && rem > 0 && (c[0] >> 3) == J;
+      }
     }
     if (FILL) {
-      T tile_row[8];
+      if (J != kNoBlock) {
+        if (l == 0) bsr_indices[out] = J;
+        T* dst = blocks + out * 64 + l * 8;
+        uint32_t w[8];
 #pragma unroll
-      for (int c = 0; c < 8; ++c) tile_row[c] = from_float<T>(0.f);
-      if (dense) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) tile_row[k] = from_float<T>(val_stage[staged(off + k)]);
-      } else {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          if (k < n) {
-            const T v = from_float<T>(val_stage[staged(off + k)]);
-#pragma unroll
-            for (int c = 0; c < 8; ++c)
-              if ((col[k] & 7) == c) tile_row[c] = v;
-          }
+        for (int k = 0; k < 8; ++k) w[k] = bits(tile_row[k]);
+        uint4* d4 = reinterpret_cast<uint4*>(dst);
+        if (sizeof(T) == 4) {
+          d4[0] = make_uint4(w[0], w[1], w[2], w[3]);
+          d4[1] = make_uint4(w[4], w[5], w[6], w[7]);
+        } else {
+          d4[0] = make_uint4(w[0] | (w[1] << 16), w[2] | (w[3] << 16), w[4] | (w[5] << 16), w[6] | (w[7] << 16));
         }
+        ++out;
       }
-      if (l == 0) bsr_indices[out] = J;
-      T* dst = blocks + out * 64 + l * 8;
-      uint32_t w[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) w[c] = bits(tile_row[c]);
-      uint4* d4 = reinterpret_cast<uint4*>(dst);
-      if (sizeof(T) == 4) {
-        d4[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        d4[1] = make_uint4(w[4], w[5], w[6], w[7]);
-      } else {
-        d4[0] = make_uint4(w[0] | (w[1] << 16), w[2] | (w[3] << 16), w[4] | (w[5] << 16), w[6] | (w[7] << 16));
-      }
-      ++out;
-    } else {
+    } else if (J != kNoBlock) {
       ++count;
     }
-    pos += n;
-    off += n;
-    have -= n;
-    last = J;
+    if (left) {   // one by one into the tile just written
+      for (; rem > 0 && (*ip >> 3) == J; ++ip, --rem) {
+        if (FILL) blocks[(out - 1) * 64 + l * 8 + (*ip & 7)] = from_float<T>(vp ? *vp++ : 1.0f);
+      }
+      load_window();
+    }
   }
   if (!FILL && l == 0 && I < Mb) bsr_indptr[I + 1] = count;
 }
