@@ -171,7 +171,7 @@ spmm_csr_ring_kernel(const int64_t* __restrict__ indptr, const int32_t* __restri
   CsrRowIds<G> ids;
   ids.init(indptr + row_begin, (int)(row_end - row_begin), base, s0, s1, g, gl);
   const int f0 = blockIdx.y * kFeatures;
-  walk_group_ring<G, CH, 4, SH, 1>(ids, false, indices + base + s0, data ? data + base + s0 : nullptr, B + f0, ldb, C + f0, ldc,
+  walk_group_ring<G, CH, 4, SH, 1, 1>(ids, false, indices + base + s0, data ? data + base + s0 : nullptr, B + f0, ldb, C + f0, ldc,
                                    min(N - f0, kFeatures), g, gl, group_bytes + w * GroupSmem<G, CH, SH>::kBytes);
 }
 

@@ -177,6 +177,11 @@ __device__ __forceinline__ uint64_t fma_pair(uint64_t a, uint64_t b, uint64_t c)
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
   return d;
 }
+__device__ __forceinline__ uint64_t add_pair(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
 __device__ __forceinline__ float2 as_floats(uint64_t v) {
   float2 f;
   asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
@@ -188,17 +193,57 @@ __device__ __forceinline__ uint64_t as_pair(uint32_t lo, uint32_t hi) {
   return v;
 }
 
-// The sum of one row, and its way to C.
-template <int G, int CH, int VEC, bool SH>
+// The sum of one row, and its way to C.  SUMS: how its terms are grouped, hence how its error grows.
+//   1  one chain, the order of the register kernels: n terms of one size leave a variance of n^2 / 2 roundings;
+//   2  the terms of a batch of four steps in a chain of their own, the batches in another: n^2 / 8;
+//   3  batches to two chains in turn: n^2 / 16 + 4 n, at every n no more than four interleaved chains leave.
+// A chain per step of a batch would do as much but has to be added up at every row change, by one group of a
+// warp while the others wait: 2^18 power-law rows at 32 features 67 us against 47 for one chain.
+template <int G, int CH, int VEC, bool SH, int SUMS>
 struct GroupSum {
   static constexpr int kPairs = CH * VEC / 2;
-  uint64_t a[kPairs];
+  uint64_t s[SUMS][kPairs];   // s[0]: the total in the end; s[SUMS - 1]: the batch (SUMS > 1); s[1]: the other chain (3)
   __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int i = 0; i < kPairs; ++i) a[i] = 0;
+    for (int p = 0; p < SUMS; ++p)
+#pragma unroll
+      for (int i = 0; i < kPairs; ++i) s[p][i] = 0;
+  }
+  __device__ __forceinline__ void end_batch(int turn) {   // turn: the chain that takes the batch
+    if constexpr (SUMS > 1) {
+#pragma unroll
+      for (int i = 0; i < kPairs; ++i) {
+        s[turn][i] = add_pair(s[turn][i], s[SUMS - 1][i]);
+        s[SUMS - 1][i] = 0;
+      }
+    }
+  }
+  // everything into s[0]; inside: terms of a batch that has not ended may be there
+  __device__ __forceinline__ void total(bool inside) {
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) {
+      if (SUMS == 3) s[0][i] = add_pair(s[0][i], s[1][i]);
+      if (SUMS > 1 && inside) s[0][i] = add_pair(s[0][i], s[SUMS - 1][i]);
+    }
+  }
+  // after total(): nothing but the total is left
+  __device__ __forceinline__ void settle() {
+    if constexpr (SUMS == 3) {
+#pragma unroll
+      for (int i = 0; i < kPairs; ++i) s[1][i] = 0;
+    }
+  }
+  // adds the total that the lane `from` further up holds, if `take`
+  __device__ __forceinline__ void join(int from, bool take, int) {
+#pragma unroll
+    for (int i = 0; i < kPairs; ++i) {
+      const uint64_t y = __shfl_down_sync(kAllLanes, (unsigned long long)s[0][i], from);
+      if (take) s[0][i] = add_pair(s[0][i], y);
+    }
   }
   // x: this lane's first chunk of the row in the ring (CH chunks, 512 bytes apart)
   __device__ __forceinline__ void add(uint64_t val, const unsigned char* x) {
+    uint64_t* a = s[SUMS - 1];
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
       if constexpr (VEC == 4) {
@@ -216,6 +261,7 @@ struct GroupSum {
   }
   // row: this lane's first feature in C; nf: features from there to the end of the row
   __device__ __forceinline__ void write(float* row, int nf, bool open) const {
+    const uint64_t* a = s[0];
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
       if (c * G * VEC < nf) {
@@ -235,9 +281,23 @@ struct GroupSum {
   }
 };
 template <int G, int VEC>
-struct GroupSum<G, 1, VEC, true> {
+struct GroupSum<G, 1, VEC, true, 1> {
   float a[4];
   __device__ __forceinline__ void zero() { a[0] = a[1] = a[2] = a[3] = 0.f; }
+  __device__ __forceinline__ void end_batch(int) {}
+  __device__ __forceinline__ void total(bool) {}
+  __device__ __forceinline__ void settle() {}
+  // h: the group that gives.  Its lanes hold the features of the group before it, one place on where the two
+  // groups start with different features.
+  __device__ __forceinline__ void join(int from, bool take, int h) {
+    const bool turned = G != 4 || (h & 1) == 0;
+    float y[4];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) y[v] = __shfl_down_sync(kAllLanes, turned ? a[(v + 3) & 3] : a[v], from);
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+      if (take) a[v] += y[v];
+  }
   // feature v of lane gl: the groups that share banks (G = 4: every other one) start with different v
   static __device__ __forceinline__ int feature(int v, int g, int gl) { return gl + G * ((v + (G == 4 ? g >> 1 : g)) & 3); }
 };
@@ -245,8 +305,9 @@ struct GroupSum<G, 1, VEC, true> {
 // One warp; cols / vals point at the calling group's first slot (vals == nullptr: all ones), `ids`
 // knows the rows of its ids.n slots (0: the group has nothing to do).  WC: row changes happen only at
 // multiples of WC slots.  all_open: every row may be held by other groups too.  C: row 0 of the output
-// the row ids count from, at the first feature of this walk; nf: features from there on.
-template <int G, int CH, int VEC, bool SH, int WC, class Rows>
+// the row ids count from, at the first feature of this walk; nf: features from there on.  The groups of
+// a warp hold neighbouring ranges.
+template <int G, int CH, int VEC, bool SH, int WC, int SUMS, class Rows>
 __device__ __forceinline__ void walk_group_ring(Rows& ids, bool all_open, const int32_t* __restrict__ cols,
                                                 const float* __restrict__ vals,
                                                 const typename BTraits<VEC>::elem* __restrict__ B, int ldb,
@@ -273,13 +334,14 @@ __device__ __forceinline__ void walk_group_ring(Rows& ids, bool all_open, const 
   const uint32_t pitch = (uint32_t)ldb * (uint32_t)sizeof(Elem), pitch_c = (uint32_t)ldc * 4u;   // checked by the launch
   const int over = SH ? gl * 16 - nf * 4 : 0;   // SH: chunk gl is needed while the shift is larger than this
 
-  GroupSum<G, CH, VEC, SH> sum;
+  GroupSum<G, CH, VEC, SH, SUMS> sum;
   sum.zero();
   int cur = ids.first;
   bool open = all_open || ids.head_open;
   float* Cl = C + (SH ? 0 : gl * VEC);
-  auto flush = [&](bool open_now) {
+  auto flush = [&](bool open_now, bool inside) {
     float* row = reinterpret_cast<float*>(const_cast<void*>(row_of_b(Cl, (uint32_t)cur, pitch_c)));
+    sum.total(inside);
     if constexpr (SH) {
 #pragma unroll
       for (int v = 0; v < 4; ++v) {
@@ -356,7 +418,7 @@ __device__ __forceinline__ void walk_group_ring(Rows& ids, bool all_open, const 
   wait_for_prior_grid();   // no store or atomic to C before the row-clearing launch is complete
 
   int cell = g * 4, half = 0;   // consumer
-  for (int j = 0; j < nmax; j += U) {
+  auto batch = [&](int j, int turn) {   // the four steps from j on
     const int4 r4 = *reinterpret_cast<const int4*>(rd + cell);
     const ulonglong2 va = *reinterpret_cast<const ulonglong2*>(sv + cell), vb = *reinterpret_cast<const ulonglong2*>(sv + cell + 2);
     const int start[U] = {r4.x, r4.y, r4.z, r4.w};
@@ -370,7 +432,7 @@ __device__ __forceinline__ void walk_group_ring(Rows& ids, bool all_open, const 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (u % WC == 0 && start[u] >= 0) {
-        flush(open);
+        flush(open, u > 0);
         cur = start[u];
         open = all_open;
       }
@@ -385,12 +447,36 @@ __device__ __forceinline__ void walk_group_ring(Rows& ids, bool all_open, const 
         if (as_floats(val[u]).x != 0.f) sum.add(val[u], x + u * (CH * 512));
       }
     }
+    sum.end_batch(turn);
     if constexpr (SH) __syncwarp();    // every lane has read before the slots are refilled
     cell = (cell + U * R) & (kCells - 1);
     half ^= kHalf;
     issue_batch(j + 2 * U);            // refills exactly the ring slots read above
+  };
+  if constexpr (SUMS == 3) {
+    for (int j = 0; j < nmax; j += 2 * U) {
+      batch(j, 0);
+      if (j + U < nmax) batch(j + U, 1);
+    }
+  } else {
+    for (int j = 0; j < nmax; j += U) batch(j, 0);
   }
-  if (n > 0) flush(open || ids.last_open());
+  // A row that goes on over whole ranges: a group that saw nothing else hands its sum to the group before it,
+  // the last one first, so that such a row costs one atomic add per warp and not one per range, and the chain
+  // of those adds is that much shorter.
+  bool give = false;
+  if constexpr (R > 1) {
+    const int before = __shfl_up_sync(kAllLanes, n > 0 ? cur : -1, G);
+    give = g > 0 && n > 0 && cur == ids.first && before == cur;
+    if (__any_sync(kAllLanes, give)) {
+      sum.total(false);
+      sum.settle();
+      for (int h = R - 1; h > 0; --h) {
+        if (__shfl_sync(kAllLanes, give, h * G)) sum.join(G, g == h - 1, h);
+      }
+    }
+  }
+  if (n > 0 && !give) flush(open || ids.last_open(), false);
 }
 
 }  // namespace lf
