@@ -152,11 +152,16 @@ spmm_csr_kernel(const int64_t* __restrict__ indptr, const int32_t* __restrict__ 
 }
 
 // The CSR product with the gathers staged through the group ring (lf_spmm_group.cuh): a group takes
-// spg consecutive entries, adds them up in the order of the register kernel above and flushes by the
-// same rules.  2^18 power-law rows, 3.7 M entries, register kernel / ring: 16 features 152 / 39 us, 64
-// features 213 / 80 us, 128 features (one row per warp and step / two) 147 / 137 us.
+// spg consecutive entries and flushes by the rules of the register kernel above.  2^18 power-law rows, 3.7 M
+// entries, register kernel / ring: 16 features 164 / 50 us, 64 features 226 / 92 us, 128 features 236 / 141 us.
+//
+// Sums in batches (2) allow ranges four times as long at no larger error; one chain (1) keeps the ranges, and the
+// order, of the register kernel.  2^19 power-law rows at 32 features: chain 130 us, batches 123; 2^18 at 64 98 / 92,
+// at 160 221 / 208; but at 16 48 / 53 and shifted at 47 146 / 150: there a range's start is cheap beside its rows.
+template <int G, bool SH> constexpr int kCsrSums = SH || G == 4 || G == 16 ? 1 : 2;
+
 template <int G, int CH, bool SH>
-__global__ void __launch_bounds__(kThreads, CH == 1 ? 4 : 3)
+__global__ void __launch_bounds__(kThreads, CH == 1 && kCsrSums<G, SH> == 1 ? 4 : 3)
 spmm_csr_ring_kernel(const int64_t* __restrict__ indptr, const int32_t* __restrict__ indices,
                      const float* __restrict__ data, int64_t row_begin, int64_t row_end,
                      const float* __restrict__ B, int ldb, float* __restrict__ C, int64_t ldc, int N, int spg) {
@@ -171,8 +176,9 @@ spmm_csr_ring_kernel(const int64_t* __restrict__ indptr, const int32_t* __restri
   CsrRowIds<G> ids;
   ids.init(indptr + row_begin, (int)(row_end - row_begin), base, s0, s1, g, gl);
   const int f0 = blockIdx.y * kFeatures;
-  walk_group_ring<G, CH, 4, SH, 1, 1>(ids, false, indices + base + s0, data ? data + base + s0 : nullptr, B + f0, ldb, C + f0, ldc,
-                                   min(N - f0, kFeatures), g, gl, group_bytes + w * GroupSmem<G, CH, SH>::kBytes);
+  walk_group_ring<G, CH, 4, SH, 1, kCsrSums<G, SH>>(ids, false, indices + base + s0, data ? data + base + s0 : nullptr,
+                                                    B + f0, ldb, C + f0, ldc, min(N - f0, kFeatures), g, gl,
+                                                    group_bytes + w * GroupSmem<G, CH, SH>::kBytes);
 }
 
 }  // namespace
@@ -211,8 +217,16 @@ int lf_spmm_csr_f32(const int64_t* indptr, const int32_t* indices, const float* 
   // search, so long ranges win as soon as the grid fills the chip about twice; measured on
   // 3.7 M entries, 16 features: 32 / 64 / 128 / 256 entries 74.8 / 68.1 / 65.4 / 63.6 us, on 1 M entries, 128
   // features 51.3 / 45.1 / 45.3 / 51.4 us.  Below that, more blocks win until a range is one strip.
-  int spg = 256;
-  while (spg > 32 && ceil_div64(nnz, (int64_t)spg * gpc) < (int64_t)sm_count() * 3 * 2) spg >>= 1;
+  // But a range is a chain of additions, and a row's error grows with it: one chain is no longer than what
+  // fills the chip eight times at cfg.G lanes per row, batches no longer than four times that.
+  int chain = 256;
+  while (chain > 32 && ceil_div64(nnz, (int64_t)chain * (kThreads / cfg.G)) < (int64_t)sm_count() * 3 * 8) chain >>= 1;
+  int spg = chain;
+  if (ring) {
+    const int longest = cfg.VEC == 4 && (group.G == 8 || group.G == 32) ? 4 * chain : chain;   // kCsrSums
+    for (spg = 256; spg > 32; spg >>= 1)
+      if (spg <= longest && ceil_div64(nnz, (int64_t)spg * gpc) >= (int64_t)sm_count() * 3 * 2) break;
+  }
   const int64_t rows = row_end - row_begin;
   {
     const int spg_log = 31 - __builtin_clz((unsigned)spg);

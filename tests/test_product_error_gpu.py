@@ -84,3 +84,17 @@ def test_long_rows(cuda_device, dtype, N, chains):
         sums[0].append(_rms(hyb.spmm_hyb(fmt, B)[:, f:f + 8], exact) ** 2)
         sums[1].append(_rms(_ranges(vals, X, 32, chains), exact) ** 2)
     assert np.mean(sums[0]) ** 0.5 <= 1.08 * np.mean(sums[1]) ** 0.5
+
+
+@pytest.mark.parametrize("N,lanes", [(32, 8), (64, 16), (128, 32), (200, 32), (47, 32), (9, 32)])
+def test_csr_rows_of_256_entries(cuda_device, N, lanes):
+    """3.7 M entries: chains of as many entries as fill the chip eight times, at 32 entries or more."""
+    import torch
+    csr, cols, vals = _matrix(14_336, 256, cuda_device, 5)
+    chain, blocks = 256, torch.cuda.get_device_properties(cuda_device).multi_processor_count * 3 * 8
+    while chain > 32 and -(-csr.nnz // (chain * (256 // lanes))) < blocks:
+        chain //= 2
+    B = _features(N, "float32", cuda_device)
+    X = B[:, :8][cols]
+    exact = (X.double() * vals.double()[:, :, None]).sum(1)
+    assert _rms(hyb.spmm_csr(csr, B)[:, :8], exact) <= 1.03 * _rms(_ranges(vals, X, chain), exact)
