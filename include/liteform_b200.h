@@ -242,6 +242,8 @@ int lf_spmm_hyb_f32(const lf_hyb* A, const float* B /*[dev] K x N*/, int64_t ldb
  * nothing.  For logs and benchmarks. */
 const char* lf_spmm_hyb_f32_kernel_name(const lf_hyb* A, const float* B, int64_t ldb, const float* C, int64_t ldc,
                                         int32_t N);
+/* The same for lf_spmm_hyb_bf16 (its operands are 16-byte aligned). */
+const char* lf_spmm_hyb_bf16_kernel_name(const lf_hyb* A, int64_t ldb, int64_t ldc, int32_t N);
 
 /* The same product with B in bf16 (raw 16-bit patterns), values and accumulation in float32, C in
  * float32: halves the bytes of every gather.  N and ldb multiples of 8, ldc of 4, B and C 16-byte

@@ -927,26 +927,38 @@ int launch_hyb(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, const
 // the registers (473 062 power-law rows, 27 features, 4 partitions: 161 us, shifted copies into a ring 212 us).
 // "Touched" is what the stored slots can reach of B; times are us, form on the other side / form taken.
 //   * By groups while that stays in the L2 beside what streams through.  2^18 power-law rows: 32 features
-//     (34 MB) 65 / 47, 64 (67 MB) 81 / 76 and with 4 partitions 121 / 103; 100 000 Zipf rows at 200 features,
-//     2 partitions (80 MB) 154 / 135; 4000 at 512 29 / 18.  Past it: 400 000 uniform rows at 64 features
+//     (34 MB) 64 / 50, 64 (67 MB) 80 / 75 and with 4 partitions 120 / 99; 100 000 Zipf rows at 200 features,
+//     2 partitions (80 MB) 153 / 146; 4000 at 512 27 / 17.  Past it: 400 000 uniform rows at 64 features
 //     (102 MB) groups 244, consecutive slots 225; 2^18 power-law rows at 100 features (105 MB) 173, ring per warp 164.
 //     Rows of up to 128 bytes, where the other form has four partial sums to add, a little longer: 2^20
-//     power-law rows at 24 features, 8 partitions (101 MB) 311 / 250; at 134 MB of uniform rows 424 against 457.
+//     power-law rows at 24 features, 8 partitions (101 MB) 310 / 253; at 134 MB of uniform rows 424 against 457.
+//     From 2^20 slots on, when the other forms fill the chip, they keep two widths: float32 rows of 65 to 128
+//     features, which fill a warp (2^17 power-law rows at 128 groups 67.5, ring per warp 64.3, with 4
+//     partitions 95.2 / 87.9, at 72 62.0 / 59.7; uniform 125.3 / 120.9; with partitions at any size: 40 000
+//     power-law rows at 128, 4 partitions 37.5 / 33.3), and bf16 rows of 65 to 128 (2^18
+//     uniform rows at 128 196, consecutive slots 180, power-law rows with 4 partitions 244 / 223).
 //     bf16 rows of more than 256 bytes keep the ring per warp (16 234 Zipf rows, 240 features: 27.4, groups 28.7).
 //   * bf16 rows of more than 256 bytes in pieces of 256 bytes, by consecutive slots, once 512-byte pieces of
-//     B are more than twice the L2: a piece finds more of itself there.  256 features: 2^20 skewed rows 1748 /
-//     1682, uniform 2318 / 1998, 2^19 power-law rows with 8 partitions 1091 / 1003.  In float32 a uniform matrix
-//     gains as much (2^20 rows at 128 features 2236 / 1915) but the power-law graph gains nothing (564 to 571
-//     either way, 648 / 665 on another card) and loses to the second reading of the slots below that size
-//     (2^18 rows at 256 features 236 / 279): float32 keeps the ring per warp.
+//     B are more than twice the L2: a piece finds more of itself there.  Only where the last piece is full, or
+//     where their number is odd, so that they save half a walk of a full warp.  256 features, ring per warp / pieces:
+//     2^19 uniform rows 981 / 804, 2^20 2314 / 2001, skewed 1703 / 1529, 2^19 power-law rows with 8 partitions
+//     1087 / 1000, 2^20 with one 720 / 748; 320 features 3566 / 2801, 2655 / 2162, 1416 / 1311, 1313 / 1120 of the last
+//     four.  A short last piece loses, the slots are read once more for it: 2^20 uniform rows at 136 / 192 / 240
+//     features 1514 / 1701 / 2532 in one walk, 2101 / 1738 / 2837 in two; power-law rows at 448 1373 / 1490.  In float32 a
+//     uniform matrix gains as much (2^20 rows at 128 features 2236 / 1915) but the power-law graph gains nothing
+//     (564 to 571 either way, 648 / 665 on another card) and loses to the second reading of the slots below that
+//     size (2^18 rows at 256 features 236 / 279): float32 keeps the ring per warp.
 Form form_of(const lf_hyb* A, const FeatCfg& cfg, int64_t ldb, int64_t ldc, int N, bool several_dests) {
   if (gather_ring() == 0 || cache_policy() != 1 || cfg.VEC == 1 || several_dests || ldb >= (1ll << 30)) return Form::kOther;
   const int64_t slots = A->slot_off[A->num_buckets], reach = A->num_cols < slots ? A->num_cols : slots;
   const int64_t row = (int64_t)N * (cfg.VEC == 8 ? 2 : 4);
   const int64_t resident = (row <= 128 ? 104ll : 80ll) << 20;
-  if (g_ring_rows_min_slots > 0 && reach * row <= resident && ldc < (1ll << 30) && (row <= 256 || cfg.VEC == 4)) return Form::kGroups;
-  if (slots < g_ring_rows_min_slots) return Form::kOther;
-  const bool pieces = (cfg.VEC == 8 && reach * 512 >= (256ll << 20)) || g_ring_rows_min_slots == 0;
+  const bool many = slots >= g_ring_rows_min_slots;
+  const bool width = cfg.VEC == 8 ? row <= (many ? 128 : 256) : row <= 256 || row > 512 || (!many && A->num_parts == 1);
+  if (g_ring_rows_min_slots > 0 && reach * row <= resident && ldc < (1ll << 30) && width) return Form::kGroups;
+  if (!many) return Form::kOther;
+  const bool full = (N + 127) / 128 % 2 == 1 || N % 128 == 0;
+  const bool pieces = (cfg.VEC == 8 && full && reach * 512 >= (256ll << 20)) || g_ring_rows_min_slots == 0;
   return row <= 256 || pieces ? Form::kSlots : Form::kOther;
 }
 
@@ -1038,16 +1050,22 @@ int lf_spmm_hyb_f32(const lf_hyb* A, const float* B, int64_t ldb, float* C, int6
   return spmm_hyb_impl(A, B, false, ldb, C, ldc, N, flags, stream, none);
 }
 
-const char* lf_spmm_hyb_f32_kernel_name(const lf_hyb* A, const float* B, int64_t ldb, const float* C, int64_t ldc,
-                                        int32_t N) {
-  if (!A || N < 1) return "";
-  const FeatCfg cfg = pick_cfg(B, ldb, C, ldc, N);
+static const char* kernel_name(const lf_hyb* A, const FeatCfg& cfg, int64_t ldb, int64_t ldc, int32_t N) {
   switch (A->slot_off ? form_of(A, cfg, ldb, ldc, N, false) : Form::kOther) {
     case Form::kGroups: return "spmm_hyb_groups_kernel";
     case Form::kSlots: return "spmm_hyb_ring_rows_kernel";   // buckets narrower than the slots of a step: spmm_hyb_kernel
     default: break;
   }
-  return gather_ring() > 0 && ring_applies(cfg, ldb) ? "spmm_hyb_ring_kernel" : "spmm_hyb_kernel";
+  return gather_ring() > 0 && cfg.VEC != 1 && cfg.G == 32 && ldb < (1ll << 30) ? "spmm_hyb_ring_kernel" : "spmm_hyb_kernel";
+}
+
+const char* lf_spmm_hyb_f32_kernel_name(const lf_hyb* A, const float* B, int64_t ldb, const float* C, int64_t ldc,
+                                        int32_t N) {
+  return !A || N < 1 ? "" : kernel_name(A, pick_cfg(B, ldb, C, ldc, N), ldb, ldc, N);
+}
+
+const char* lf_spmm_hyb_bf16_kernel_name(const lf_hyb* A, int64_t ldb, int64_t ldc, int32_t N) {
+  return !A || N < 1 ? "" : kernel_name(A, pick_cfg_bf16(N), ldb, ldc, N);
 }
 
 int lf_spmm_hyb_bf16(const lf_hyb* A, const uint16_t* B, int64_t ldb, float* C, int64_t ldc, int32_t N,

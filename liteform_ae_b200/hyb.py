@@ -351,11 +351,12 @@ def spmm_hyb(fmt: HybFormat, B, out=None, accumulate: bool = False):
 
 
 def spmm_hyb_kernel_name(fmt: HybFormat, B, out) -> str:
-    """``lf_spmm_hyb_f32_kernel_name``: the kernel ``spmm_hyb(fmt, B, out=out)`` launches for float32 B."""
-    s = fmt.c_struct()
-    name = _cabi.load().lf_spmm_hyb_f32_kernel_name(C.byref(s), B.data_ptr(), B.stride(0), out.data_ptr(),
-                                                    out.stride(0), int(B.shape[1]))
-    return name.decode()
+    """``lf_spmm_hyb_f32_kernel_name`` / ``lf_spmm_hyb_bf16_kernel_name``: the kernel that
+    ``spmm_hyb(fmt, B, out=out)`` launches."""
+    lib, s, N = _cabi.load(), fmt.c_struct(), int(B.shape[1])
+    if B.dtype == _torch().bfloat16:
+        return lib.lf_spmm_hyb_bf16_kernel_name(C.byref(s), B.stride(0), out.stride(0), N).decode()
+    return lib.lf_spmm_hyb_f32_kernel_name(C.byref(s), B.data_ptr(), B.stride(0), out.data_ptr(), out.stride(0), N).decode()
 
 
 def spmm_csr(csr: DeviceCsr, B, out=None, row_range=None):

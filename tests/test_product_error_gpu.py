@@ -66,7 +66,7 @@ def test_rows_of_one_ell_row(cuda_device, n, dtype, N, chains):
     X = B[:, :8].float()[cols]
     exact = (X.double() * vals.double()[:, :, None]).sum(1)
     got = hyb.spmm_hyb(fmt, B)
-    if dtype == "float32":
+    if dtype == "float32" and N <= 64:
         assert hyb.spmm_hyb_kernel_name(fmt, B, got) == "spmm_hyb_groups_kernel"
     assert _rms(got[:, :8], exact) <= 1.03 * _rms(_interleaved(vals, X, chains), exact)
 

@@ -1,5 +1,5 @@
 """The composed-format product on both sides of every line of the rule that picks its kernel: rows of B
-around 128 and 256 bytes, a B that stays in the L2 and one that does not, more columns than 512-byte pieces
+around 128 and 256 bytes, a B that stays in the L2 and one that does not, more columns than 512-byte rows
 are taken whole for, buckets narrower than a step, rows cut by groups, one and two partitions.
 
 Tolerance: the float32 product's (rel 1e-5 / abs 1e-4 against float64; no row has more than 600 entries)."""
@@ -8,7 +8,7 @@ import pytest
 from liteform_ae_b200 import _cabi, hyb
 
 pytestmark = pytest.mark.gpu
-M = 9000
+M = 12000
 
 
 @pytest.fixture(scope="module", params=[30_000, 300_000, (1 << 19) + 8])
@@ -32,7 +32,7 @@ def matrix(request, cuda_device):
 
 
 @pytest.mark.parametrize("dtype,N", [("float32", n) for n in (4, 28, 32, 36, 64, 68, 72, 128, 132)] +
-                         [("bfloat16", n) for n in (8, 64, 72, 128, 136, 264)])
+                         [("bfloat16", n) for n in (8, 64, 72, 128, 136, 248, 256, 264)])
 def test_forms(matrix, cuda_device, dtype, N):
     import torch
     csr, rows, formats = matrix
@@ -49,10 +49,16 @@ def test_forms(matrix, cuda_device, dtype, N):
         C = torch.ones((M, N), device=cuda_device)
         hyb.spmm_hyb(fmt, B, out=C, accumulate=True)
         torch.testing.assert_close(C.double(), want + 1, rtol=1e-5, atol=2e-4)
-    if dtype == "float32":
-        row, reach = 4 * N, min(K, int(formats[0].total_slots))
-        if reach * row <= (104 if row <= 128 else 80) << 20:
+    for fmt in formats:
+        row, slots = N * (4 if dtype == "float32" else 2), int(fmt.slot_off[-1])
+        reach = min(K, slots)
+        fits = reach * row <= (104 if row <= 128 else 80) << 20
+        if fits and (row <= 128 or (dtype == "float32" and (row <= 256 or row > 512))):   # 65 to 128 features: many slots
             name = "spmm_hyb_groups_kernel"
+        elif row <= 256 or (dtype == "bfloat16" and N >= 256 and reach >= 1 << 19):
+            name = "spmm_hyb_ring_rows_kernel"
         else:
-            name = "spmm_hyb_ring_rows_kernel" if row <= 256 else "spmm_hyb_ring_kernel"
-        assert hyb.spmm_hyb_kernel_name(formats[0], B, C) == name
+            name = "spmm_hyb_ring_kernel"
+        assert hyb.spmm_hyb_kernel_name(fmt, B, C) == name
+    if K > 1 << 19:    # both ways of a wide bf16 row are reached, with plain stores and with atomic adds
+        assert min(int(f.slot_off[-1]) for f in formats) >= 1 << 19
