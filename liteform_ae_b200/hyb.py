@@ -154,16 +154,23 @@ class HybFormat:
         self.__dict__[name] = value
         self.__dict__["_c_view"] = None      # any attribute may be part of the C view kept below
 
+    def __delattr__(self, name):
+        super().__delattr__(name)
+        self.__dict__["_c_view"] = None
+
     def __getstate__(self):
         return {k: v for k, v in self.__dict__.items() if k != "_c_view"}
 
     def _c_ref(self):
-        """``byref`` of ``c_struct()``, kept until an attribute is assigned or a device array changes its
-        address: filling the structure costs more host time than a small product takes on the device."""
-        z = self.zero_rows
-        now = (self.rows.data_ptr(), self.cols.data_ptr(), self.vals.data_ptr(), -1 if z is None else z.data_ptr())
+        """``byref`` of ``c_struct()`` for a product, which does not read ``mask``.  Kept until an attribute is
+        assigned or deleted, or a device array is given another address, strides or number of rows to clear in
+        place: filling the structure costs more host time than a small product takes on the device."""
+        r, c, v, z = self.rows, self.cols, self.vals, self.zero_rows
+        if r is None or c is None or v is None:
+            return C.byref(self.c_struct())
+        now = (r.data_ptr(), c.data_ptr(), v.data_ptr(), None if z is None else (z.data_ptr(), z.numel()))
         kept = self.__dict__.get("_c_view")
-        if kept is None or kept[0] != now:
+        if kept is None or kept[0] != now or not (r.is_contiguous() and c.is_contiguous() and v.is_contiguous()):
             s = self.c_struct()
             kept = (now, C.byref(s), s)
             self.__dict__["_c_view"] = kept
