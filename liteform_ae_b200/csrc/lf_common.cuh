@@ -6,9 +6,6 @@
 #include <stdio.h>
 #include <stdarg.h>
 
-#include <atomic>
-#include <mutex>
-
 #include "liteform_b200.h"
 
 namespace lf {
@@ -36,22 +33,12 @@ constexpr int kBucketAlign = 64;  // elements; bucket starts inside the rows/col
 
 __host__ __device__ inline int64_t ceil_div64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-// Raises a kernel's dynamic shared-memory limit, once per device and size: the attribute call takes
-// about as long as a tenth of a launch and would otherwise precede every product.
+// Raises a kernel's dynamic shared-memory limit.  The limit belongs to the kernel in the current context, and a
+// process may have several on a device or reset it, so it is set before every launch (no difference in a
+// product of 14 us).
 template <auto Kernel>
 inline cudaError_t allow_smem(int bytes) {
-  constexpr int kMaxDevices = 64;
-  static std::atomic<int> have[kMaxDevices];
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  if (dev < kMaxDevices && have[dev].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
-  static std::mutex lock;   // a smaller request must not come after a larger one
-  std::lock_guard<std::mutex> guard(lock);
-  if (dev < kMaxDevices && have[dev].load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
-  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess && dev < kMaxDevices) have[dev].store(bytes, std::memory_order_release);
-  return e;
+  return cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 
 // ceil(log2(d)) for d >= 1, on integers (the reference uses math.ceil(math.log2(d))).
