@@ -765,7 +765,8 @@ def roofline_of(prob, rec, world):
             "gather_model_bytes_per_clk_per_sm": gath / (launch_ms * 1e-3) / (148 * world * 1.965e9)}
 
 
-KERNEL_SOURCES = {"hyb": ("lf_spmm_hyb.cu", "lf_common.cuh"), "bsr8": ("lf_spmm_bsr8.cu", "lf_bsr8_mma.cuh")}
+KERNEL_SOURCES = {"hyb": ("lf_spmm_hyb.cu", "lf_spmm_group.cuh", "lf_spmm_gather.cuh", "lf_bsr8_tma.cuh", "lf_common.cuh"),
+                  "bsr8": ("lf_spmm_bsr8.cu", "lf_bsr8_mma.cuh", "lf_bsr8_tma.cuh", "lf_common.cuh")}
 
 
 def kernel_source_hash(family):

@@ -31,3 +31,20 @@ def test_reference_arm_prints_the_contract_line():
 def test_reference_arm_other_ranks_stay_silent():
     res = _run({"RANK": "1", "LOCAL_RANK": "1", "WORLD_SIZE": "2"})
     assert res.returncode == 0 and res.stdout.strip() == ""
+
+
+def test_traffic_figures_are_tied_to_every_file_of_a_kernel():
+    """The hash behind a captured figure covers the kernel's source and every header of csrc/ that it includes."""
+    import re
+    sys.path.insert(0, ROOT)
+    import bench
+    csrc = os.path.join(ROOT, "liteform_ae_b200", "csrc")
+
+    def includes(name, seen):
+        for h in re.findall(r'#include "([^"]+)"', open(os.path.join(csrc, name)).read()):
+            if h not in seen and os.path.exists(os.path.join(csrc, h)):
+                seen.add(h)
+                includes(h, seen)
+        return seen
+    for files in bench.KERNEL_SOURCES.values():
+        assert set(files) == {files[0]} | includes(files[0], set())
