@@ -65,13 +65,14 @@ inline GroupCfg pick_group_shifted(int N) {
 }
 template <int G, int CH, int VEC, bool SH> constexpr int kGroupFeatures = SH ? 4 * G - 4 : G * CH * VEC;
 
-// Shared memory of one warp: the ring, then value pairs, columns and row starts of the strips, then
-// (SH) the shifts in bytes and a few words that a shifted read past the row's end may touch.
+// Shared memory of one warp: the ring, then value pairs, columns and row starts of the strips, then (SH) the
+// shifts in bytes.  A shifted read past the row's end takes words of the next row, at the end of the ring of
+// the value pairs behind it; the sums that get them have no feature and are dropped.
 template <int G, int CH, bool SH>
 struct GroupSmem {
   static constexpr int kCells = kGroupStrips<G> * 32;
   static constexpr int kRing = kGroupSteps * CH * 512;
-  static constexpr int kBytes = kRing + kCells * 16 + (SH ? kCells * 4 + 16 : 0);
+  static constexpr int kBytes = kRing + kCells * 16 + (SH ? kCells * 4 : 0);
   static_assert(kBytes % 16 == 0, "the next warp's ring starts on a 16-byte boundary");
 };
 
