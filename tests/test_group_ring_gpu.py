@@ -1,4 +1,4 @@
-"""The gather ring for groups of 8, 16 and 32 lanes at the sizes where it can go wrong: feature counts
+"""The gather ring for groups of 4, 8, 16 and 32 lanes at the sizes where it can go wrong: feature counts
 around the capacity of a group (4 G aligned, 4 G - 4 not), row changes at every place of a strip, runs
 of empty rows longer than a strip, rows cut by group boundaries, operands off the 16-byte grid.
 
@@ -24,12 +24,14 @@ def _matrix():
     return synth.Csr(indptr, indices, rng.uniform(-1, 1, len(indices)).astype(np.float32), (len(lens), K))
 
 
-@pytest.fixture(scope="module")
-def setup(cuda_device):
+@pytest.fixture(scope="module", params=[1 << 20, 0], ids=["groups", "slots"])
+def setup(request, cuda_device):
+    """The composed-format product by groups of lanes (a small product) and, with a threshold of 0, by consecutive
+    slots per step; the CSR product has the group ring alone."""
     csr = _matrix()
     d = hyb.DeviceCsr.from_host(csr.indptr, csr.indices, csr.data, csr.shape, cuda_device)
     lib = _cabi.load()
-    assert lib.lf_set_option(_cabi.LF_OPT_SPMM_RING_MIN_SLOTS, 0) == 0     # the ring form for small products too
+    assert lib.lf_set_option(_cabi.LF_OPT_SPMM_RING_MIN_SLOTS, request.param) == 0
     yield csr, d, hyb.build_hyb_device(d, [[1, 2, 4, 16, 64]], with_mask=False), csr.toscipy().astype(np.float64)
     lib.lf_set_option(_cabi.LF_OPT_SPMM_RING_MIN_SLOTS, 1 << 20)
 
@@ -49,6 +51,30 @@ def test_products_around_the_group_capacity(setup, cuda_device, N):
                 got = C.cpu().numpy()
                 np.testing.assert_allclose(got[:, 2:2 + N], want, rtol=1e-5, atol=1e-4)
                 assert np.isnan(got[:, :2]).all() and np.isnan(got[:, 2 + N:]).all()
+
+
+@pytest.mark.parametrize("dtype,N", [("float32", n) for n in (4, 12, 16, 20, 28, 32, 36, 48, 60, 64, 68, 100, 124, 128, 132, 256, 260)] +
+                         [("bfloat16", n) for n in (8, 32, 40, 64, 72, 120, 128)])
+def test_operands_on_the_16_byte_grid(request, setup, cuda_device, dtype, N):
+    """Contiguous operands and column windows of wider ones, C written and added to, next to untouched columns."""
+    import torch
+    csr, d, fmt, A = setup
+    slots = "slots" in request.node.callspec.id.split("-")
+    wide = torch.from_numpy(synth.dense_features(K, N + 16, 5)).to(cuda_device).to(getattr(torch, dtype))
+    for B in (wide[:, 8:8 + N], wide[:, 8:8 + N].contiguous()):
+        want = A @ B.float().cpu().numpy().astype(np.float64)
+        C = torch.full((csr.shape[0], N + 8), float("nan"), device=cuda_device)
+        out = C[:, 4:4 + N]
+        assert hyb.spmm_hyb_kernel_name(fmt, B, out) == ("spmm_hyb_ring_rows_kernel" if slots else "spmm_hyb_groups_kernel")
+        hyb.spmm_hyb(fmt, B, out=out)
+        np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-5, atol=1e-4)
+        hyb.spmm_hyb(fmt, B, out=out, accumulate=True)
+        np.testing.assert_allclose(out.cpu().numpy(), 2 * want, rtol=1e-5, atol=2e-4)
+        if dtype == "float32":
+            out.fill_(float("nan"))
+            hyb.spmm_csr(d, B, out=out)
+            np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-5, atol=1e-4)
+        assert torch.isnan(C[:, :4]).all() and torch.isnan(C[:, 4 + N:]).all()
 
 
 @pytest.mark.parametrize("N", [32, 47, 64, 128])

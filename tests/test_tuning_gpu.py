@@ -151,7 +151,8 @@ def test_ring_kernels_with_strided_operands(cuda_device, restore_defaults, N):
 
 @pytest.mark.parametrize("N", [100, 128, 384])
 def test_csr_product_with_and_without_the_gather_ring(cuda_device, restore_defaults, N):
-    """lf_spmm_csr_f32 has the same two forms; rows that one thread group owns are bit-identical."""
+    """lf_spmm_csr_f32 with its gathers in a ring and in registers; rows that one thread group owns are
+    bit-identical at these widths."""
     import torch
     lib = _cabi.load()
     csr = synth.skewed_rows(M=6000, seed=9, heavy_rows=4, heavy_len=2000)
