@@ -153,18 +153,22 @@ spmm_csr_kernel(const int64_t* __restrict__ indptr, const int32_t* __restrict__ 
 
 // The CSR product with the gathers staged through the group ring (lf_spmm_group.cuh): a group takes
 // spg consecutive entries and flushes by the rules of the register kernel above.  2^18 power-law rows, 3.7 M
-// entries, register kernel / ring: 16 features 164 / 50 us, 64 features 226 / 92 us, 128 features 236 / 141 us.
+// entries, register kernel / ring: 16 features 164 / 50 us, 64 features 225 / 93 us, 128 features 235 / 137 us.
 //
-// Sums in batches (2) allow ranges four times as long at no larger error; one chain (1) keeps the ranges, and the
-// order, of the register kernel.  2^19 power-law rows at 32 features: chain 130 us, batches 123; 2^18 at 64 98 / 92,
-// at 160 221 / 208; but at 16 48 / 53 and shifted at 47 146 / 150: there a range's start is cheap beside its rows.
-template <int G, bool SH> constexpr int kCsrSums = SH || G == 4 || G == 16 ? 1 : 2;
+// Two levels (2): chains as long as the register kernel's ranges, which add up into the row's sum, so that a
+// range can hold several of them; a row inside one chain has the register kernel's sum, bit for bit.  The second
+// sum costs registers: at 64 a thread and four blocks per SM 2^19 power-law rows at 32 features take 139 us, at
+// 74 and three blocks 124, with one level 130 (and 114 with ranges of one chain of 128, 1.3 times the error);
+// 2^17 rows at 384 features one level 227, two 204.  One level where a range's start is cheap beside its rows: up to
+// 16 features (2^18 rows 48 / 53) and shifted rows (47 features 146 / 150).
+template <int G, bool SH> constexpr int kCsrSums = SH || G == 4 ? 1 : 2;
 
 template <int G, int CH, bool SH>
 __global__ void __launch_bounds__(kThreads, CH == 1 && kCsrSums<G, SH> == 1 ? 4 : 3)
 spmm_csr_ring_kernel(const int64_t* __restrict__ indptr, const int32_t* __restrict__ indices,
                      const float* __restrict__ data, int64_t row_begin, int64_t row_end,
-                     const float* __restrict__ B, int ldb, float* __restrict__ C, int64_t ldc, int N, int spg) {
+                     const float* __restrict__ B, int ldb, float* __restrict__ C, int64_t ldc, int N, int spg,
+                     int chain) {
   extern __shared__ __align__(16) unsigned char group_bytes[];
   constexpr int R = 32 / G, kFeatures = kGroupFeatures<G, CH, 4, SH>;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane / G, gl = lane % G;
@@ -176,9 +180,9 @@ spmm_csr_ring_kernel(const int64_t* __restrict__ indptr, const int32_t* __restri
   CsrRowIds<G> ids;
   ids.init(indptr + row_begin, (int)(row_end - row_begin), base, s0, s1, g, gl);
   const int f0 = blockIdx.y * kFeatures;
-  walk_group_ring<G, CH, 4, SH, 1, kCsrSums<G, SH>>(ids, false, indices + base + s0, data ? data + base + s0 : nullptr,
+  walk_group_ring<G, CH, 4, SH, 1, kCsrSums<G, SH>, 0>(ids, false, indices + base + s0, data ? data + base + s0 : nullptr,
                                                     B + f0, ldb, C + f0, ldc, min(N - f0, kFeatures), g, gl,
-                                                    group_bytes + w * GroupSmem<G, CH, SH>::kBytes);
+                                                    group_bytes + w * GroupSmem<G, CH, SH>::kBytes, chain);
 }
 
 }  // namespace
@@ -217,15 +221,17 @@ int lf_spmm_csr_f32(const int64_t* indptr, const int32_t* indices, const float* 
   // search, so long ranges win as soon as the grid fills the chip about twice; measured on
   // 3.7 M entries, 16 features: 32 / 64 / 128 / 256 entries 74.8 / 68.1 / 65.4 / 63.6 us, on 1 M entries, 128
   // features 51.3 / 45.1 / 45.3 / 51.4 us.  Below that, more blocks win until a range is one strip.
-  // But a range is a chain of additions, and a row's error grows with it: one chain is no longer than what
-  // fills the chip eight times at cfg.G lanes per row, batches no longer than four times that.
+  // But a row's error grows with the chain of additions it is summed in: a chain is no longer than the range
+  // that fills the chip eight times at cfg.G lanes per row.  Where the sum has two levels (kCsrSums), a range is
+  // several chains.
   int chain = 256;
   while (chain > 32 && ceil_div64(nnz, (int64_t)chain * (kThreads / cfg.G)) < (int64_t)sm_count() * 3 * 8) chain >>= 1;
   int spg = chain;
   if (ring) {
-    const int longest = cfg.VEC == 4 && (group.G == 8 || group.G == 32) ? 4 * chain : chain;   // kCsrSums
+    const int longest = cfg.VEC == 4 && group.G > 4 ? 256 : chain;
     for (spg = 256; spg > 32; spg >>= 1)
       if (spg <= longest && ceil_div64(nnz, (int64_t)spg * gpc) >= (int64_t)sm_count() * 3 * 2) break;
+    if (chain > spg) chain = spg;
   }
   const int64_t rows = row_end - row_begin;
   {
@@ -247,7 +253,7 @@ int lf_spmm_csr_f32(const int64_t* indptr, const int32_t* indices, const float* 
     constexpr int smem = kThreads / 32 * GroupSmem<G_, CH_, SH_>::kBytes;                                       \
     LF_CUDA_CHECK(allow_smem<kern>(smem));                                                                      \
     LF_CUDA_CHECK(launch_dep_smem(kern, rgrid, kThreads, smem, st, true, indptr, indices, data, row_begin, row_end, \
-                                  B, (int)ldb, C, ldc, N, spg));                                                \
+                                  B, (int)ldb, C, ldc, N, spg, chain));                                         \
     return LF_OK;                                                                                               \
   } while (0)
     if (cfg.VEC == 4) {

@@ -196,7 +196,8 @@ __device__ __forceinline__ uint64_t as_pair(uint32_t lo, uint32_t hi) {
 
 // The sum of one row, and its way to C.  SUMS: how its terms are grouped, hence how its error grows.
 //   1  one chain, the order of the register kernels: n terms of one size leave a variance of n^2 / 2 roundings;
-//   2  the terms of a batch of four steps in a chain of their own, the batches in another: n^2 / 8;
+//   2  the terms between two ends of a batch in a chain of their own, the batches in another: with four of them a
+//      batch, n^2 / 8;
 //   3  batches to two chains in turn: n^2 / 16 + 4 n, at every n no more than four interleaved chains leave.
 // A chain per step of a batch would do as much but has to be added up at every row change, by one group of a
 // warp while the others wait: 2^18 power-law rows at 32 features 67 us against 47 for one chain.
@@ -229,10 +230,10 @@ struct GroupSum {
   }
   // after total(): nothing but the total is left
   __device__ __forceinline__ void settle() {
-    if constexpr (SUMS == 3) {
 #pragma unroll
-      for (int i = 0; i < kPairs; ++i) s[1][i] = 0;
-    }
+    for (int p = 1; p < SUMS; ++p)
+#pragma unroll
+      for (int i = 0; i < kPairs; ++i) s[p][i] = 0;
   }
   // adds the total that the lane `from` further up holds, if `take`
   __device__ __forceinline__ void join(int from, bool take, int) {
@@ -307,17 +308,19 @@ struct GroupSum<G, 1, VEC, true, 1> {
 // knows the rows of its ids.n slots (0: the group has nothing to do).  WC: row changes happen only at
 // multiples of WC slots.  all_open: every row may be held by other groups too.  C: row 0 of the output
 // the row ids count from, at the first feature of this walk; nf: features from there on.  The groups of
-// a warp hold neighbouring ranges.
-template <int G, int CH, int VEC, bool SH, int WC, int SUMS, class Rows>
+// a warp hold neighbouring ranges.  BATCH: steps to a batch of the sums, 0: as many as `chain` (a power of two)
+// says.
+template <int G, int CH, int VEC, bool SH, int WC, int SUMS, int BATCH, class Rows>
 __device__ __forceinline__ void walk_group_ring(Rows& ids, bool all_open, const int32_t* __restrict__ cols,
                                                 const float* __restrict__ vals,
                                                 const typename BTraits<VEC>::elem* __restrict__ B, int ldb,
                                                 float* __restrict__ C, int64_t ldc, int nf, int g, int gl,
-                                                unsigned char* smem) {
+                                                unsigned char* smem, int chain = 0) {
   using Elem = typename BTraits<VEC>::elem;
   using Smem = GroupSmem<G, CH, SH>;
   constexpr int U = 4, R = 32 / G, kCells = Smem::kCells, kHalf = U * CH * 512;
   static_assert(kGroupSteps == 2 * U && G % U == 0, "two commit groups of four steps in flight");
+  static_assert(BATCH == 0 || BATCH == U, "the steps of a loop turn, or a number of turns");
   static_assert(!SH || (VEC == 4 && CH == 1), "the shifted form is for float32 rows, one chunk per lane");
   uint64_t* sv = reinterpret_cast<uint64_t*>(smem + Smem::kRing);   // {value, value}
   uint32_t* so = reinterpret_cast<uint32_t*>(sv + kCells);          // column or kNoGather
@@ -433,7 +436,7 @@ __device__ __forceinline__ void walk_group_ring(Rows& ids, bool all_open, const 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (u % WC == 0 && start[u] >= 0) {
-        flush(open, u > 0);
+        flush(open, u > 0 || BATCH == 0);
         cur = start[u];
         open = all_open;
       }
@@ -448,7 +451,7 @@ __device__ __forceinline__ void walk_group_ring(Rows& ids, bool all_open, const 
         if (as_floats(val[u]).x != 0.f) sum.add(val[u], x + u * (CH * 512));
       }
     }
-    sum.end_batch(turn);
+    if (BATCH == U || ((j + U) & (chain - 1)) == 0) sum.end_batch(turn);
     if constexpr (SH) __syncwarp();    // every lane has read before the slots are refilled
     cell = (cell + U * R) & (kCells - 1);
     half ^= kHalf;
@@ -470,14 +473,14 @@ __device__ __forceinline__ void walk_group_ring(Rows& ids, bool all_open, const 
     const int before = __shfl_up_sync(kAllLanes, n > 0 ? cur : -1, G);
     give = g > 0 && n > 0 && cur == ids.first && before == cur;
     if (__any_sync(kAllLanes, give)) {
-      sum.total(false);
+      sum.total(BATCH == 0);
       sum.settle();
       for (int h = R - 1; h > 0; --h) {
         if (__shfl_sync(kAllLanes, give, h * G)) sum.join(G, g == h - 1, h);
       }
     }
   }
-  if (n > 0 && !give) flush(open || ids.last_open(), false);
+  if (n > 0 && !give) flush(open || ids.last_open(), BATCH == 0);
 }
 
 }  // namespace lf

@@ -663,7 +663,7 @@ spmm_hyb_groups_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int32_
   ids.init(rows_arena + d.row_off, wlog, e0, e1, d.ell_rows);
   const int f0 = blockIdx.y * kFeatures;
 #define LF_WALK(WC_)                                                                                            \
-  walk_group_ring<G, CH, VEC, false, WC_, kGroupSums<G, CH>>(                                                   \
+  walk_group_ring<G, CH, VEC, false, WC_, kGroupSums<G, CH>, 4>(                                                 \
       ids, d.force_atomic != 0, cols_arena + at, vals_arena + at, B + f0, ldb, C - row_base * ldc + f0, ldc,    \
       min(N - f0, kFeatures), g, gl, ring_bytes + w * GroupSmem<G, CH, false>::kBytes)
   if (wlog == 0) LF_WALK(1);
