@@ -350,10 +350,16 @@ def spmm_hyb(fmt: HybFormat, B, out=None, accumulate: bool = False):
     else:
         assert out.shape == (n_rows, N) and out.stride(1) == 1 and out.dtype == torch.float32
     dev = B.get_device()
-    with on_device(dev):
-        fn = lib.lf_spmm_hyb_f32 if dtype is torch.float32 else lib.lf_spmm_hyb_bf16
-        check(fn(fmt._c_ref(), B.data_ptr(), B.stride(0), out.data_ptr(), out.stride(0), N,
-                 _cabi.LF_SPMM_ACCUMULATE if accumulate else _cabi.LF_SPMM_OVERWRITE, stream_of(dev)))
+    fn = lib.lf_spmm_hyb_f32 if dtype is torch.float32 else lib.lf_spmm_hyb_bf16
+    call = (fmt._c_ref(), B.data_ptr(), B.stride(0), out.data_ptr(), out.stride(0), N,
+            _cabi.LF_SPMM_ACCUMULATE if accumulate else _cabi.LF_SPMM_OVERWRITE, stream_of(dev))
+    if torch._C._cuda_getDevice() == dev:
+        status = fn(*call)
+    else:
+        with torch.cuda.device(dev):
+            status = fn(*call)
+    if status:
+        check(status)
     return out
 
 
