@@ -641,14 +641,18 @@ spmm_hyb_ring_rows_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int
 // keep four partial sums per row of up to 32 float32 (64 bf16) features, two up to 64 (128), one beyond.
 // Batches cost registers: 32 features, at most 64 registers a thread / 80, three blocks per SM: 2^18
 // power-law rows 60 / 50 us, uniform rows 110 / 89 (one chain, error 1.3 to 2 times as large: 47, 85).
-template <int G, int CH> constexpr int kGroupSums = G == 16 ? 1 : (CH == 1 ? 3 : 2);
+// Rows of more than 64 features have two levels: chains of `chain` slots, the ranges of the ring per warp, in
+// ranges that may be longer where there are blocks along y: 80 000 power-law rows at 256 features, one level
+// 86.5 us, two 79.7; 100 000 Zipf rows at 200 with 2 partitions 146, 135.
+template <int G, int CH> constexpr int kGroupSums = CH == 1 ? 3 : 2;
+template <int G> constexpr int kGroupBatch = G == 16 ? 0 : 4;
 
 template <int G, int CH, int VEC, int MAXB>
 __global__ void __launch_bounds__(kThreads, 3)
 spmm_hyb_groups_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int32_t* __restrict__ rows_arena,
                        const int32_t* __restrict__ cols_arena, const float* __restrict__ vals_arena,
                        const typename BTraits<VEC>::elem* __restrict__ B, int ldb, float* __restrict__ C, int64_t ldc,
-                       int N, int64_t row_base) {
+                       int N, int64_t row_base, int chain) {
   extern __shared__ __align__(16) unsigned char ring_bytes[];
   constexpr int R = 32 / G, GPC = kThreads / G, kFeatures = kGroupFeatures<G, CH, VEC, false>;
   int64_t tile;
@@ -663,9 +667,9 @@ spmm_hyb_groups_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int32_
   ids.init(rows_arena + d.row_off, wlog, e0, e1, d.ell_rows);
   const int f0 = blockIdx.y * kFeatures;
 #define LF_WALK(WC_)                                                                                            \
-  walk_group_ring<G, CH, VEC, false, WC_, kGroupSums<G, CH>, 4>(                                                 \
+  walk_group_ring<G, CH, VEC, false, WC_, kGroupSums<G, CH>, kGroupBatch<G>>(                                                 \
       ids, d.force_atomic != 0, cols_arena + at, vals_arena + at, B + f0, ldb, C - row_base * ldc + f0, ldc,    \
-      min(N - f0, kFeatures), g, gl, ring_bytes + w * GroupSmem<G, CH, false>::kBytes)
+      min(N - f0, kFeatures), g, gl, ring_bytes + w * GroupSmem<G, CH, false>::kBytes, max(chain, 1 << wlog))
   if (wlog == 0) LF_WALK(1);
   else if (wlog == 1) LF_WALK(2);
   else LF_WALK(4);
@@ -862,7 +866,7 @@ int launch_hyb_ring_rows(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb
 // A row of B per group of lanes.
 template <int MAXB, int VEC>
 int launch_hyb_groups(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, const void* B, int64_t ldb, float* C,
-                      int64_t ldc, int N, GroupCfg group, cudaStream_t st, bool dep) {
+                      int64_t ldc, int N, GroupCfg group, int chain, cudaStream_t st, bool dep) {
   const dim3 grid((unsigned)tiles, (unsigned)group.passes);
 #define LF_GROUPS(G_, CH_)                                                                                      \
   do {                                                                                                          \
@@ -870,7 +874,7 @@ int launch_hyb_groups(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A
     constexpr int smem = kThreads / 32 * GroupSmem<G_, CH_, false>::kBytes;                                     \
     LF_CUDA_CHECK(allow_smem<kern>(smem));                                                                      \
     LF_CUDA_CHECK(launch_dep_smem(kern, grid, kThreads, smem, st, dep, tbl, A->rows, A->cols, A->vals,          \
-                                  (const typename BTraits<VEC>::elem*)B, (int)ldb, C, ldc, N, A->row_begin));   \
+                                  (const typename BTraits<VEC>::elem*)B, (int)ldb, C, ldc, N, A->row_begin, chain)); \
     return LF_OK;                                                                                               \
   } while (0)
   if (group.G == 4) LF_GROUPS(4, 1);
@@ -887,10 +891,10 @@ enum class Form { kGroups, kSlots, kOther };
 
 template <int MAXB>
 int launch_hyb(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, const void* Bv, int64_t ldb,
-               float* C, int64_t ldc, int N, FeatCfg cfg, Form form, GroupCfg group, cudaStream_t st,
+               float* C, int64_t ldc, int N, FeatCfg cfg, Form form, GroupCfg group, int chain, cudaStream_t st,
                const DestList& dests, bool dep) {
-  if (form == Form::kGroups && cfg.VEC == 8) return launch_hyb_groups<MAXB, 8>(tbl, tiles, A, Bv, ldb, C, ldc, N, group, st, dep);
-  if (form == Form::kGroups) return launch_hyb_groups<MAXB, 4>(tbl, tiles, A, Bv, ldb, C, ldc, N, group, st, dep);
+  if (form == Form::kGroups && cfg.VEC == 8) return launch_hyb_groups<MAXB, 8>(tbl, tiles, A, Bv, ldb, C, ldc, N, group, chain, st, dep);
+  if (form == Form::kGroups) return launch_hyb_groups<MAXB, 4>(tbl, tiles, A, Bv, ldb, C, ldc, N, group, chain, st, dep);
   if (form == Form::kSlots) return launch_hyb_ring_rows<MAXB>(tbl, tiles, A, Bv, cfg.VEC == 8, ldb, C, ldc, N, cfg.G, st, dep);
   if (cfg.VEC == 8)   // bf16 B: one compiled variant per feature layout
     return launch_hyb_bf16<MAXB>(tbl, tiles, A, (const uint16_t*)Bv, ldb, C, ldc, N, cfg, st, dests, dep);
@@ -928,7 +932,7 @@ int launch_hyb(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, const
 // "Touched" is what the stored slots can reach of B; times are us, form on the other side / form taken.
 //   * By groups while that stays in the L2 beside what streams through.  2^18 power-law rows: 32 features
 //     (34 MB) 64 / 50, 64 (67 MB) 80 / 75 and with 4 partitions 120 / 99; 100 000 Zipf rows at 200 features,
-//     2 partitions (80 MB) 153 / 146; 4000 at 512 27 / 17.  Past it: 400 000 uniform rows at 64 features
+//     2 partitions (80 MB) 153 / 135; 4000 at 512 27 / 17.  Past it: 400 000 uniform rows at 64 features
 //     (102 MB) groups 244, consecutive slots 225; 2^18 power-law rows at 100 features (105 MB) 173, ring per warp 164.
 //     Rows of up to 128 bytes, where the other form has four partial sums to add, a little longer: 2^20
 //     power-law rows at 24 features, 8 partitions (101 MB) 310 / 253; at 134 MB of uniform rows 424 against 457.
@@ -1154,21 +1158,27 @@ static int spmm_hyb_impl(const lf_hyb* A, const void* B, bool b_is_bf16, int64_t
       return form != Form::kSlots || (A->widths[k] >= rows_per_step) == (pass == 0);
     };
     // A block of the group form takes up to 16384 slots: four waves of blocks are enough (2^18 power-law
-    // rows, 64 features, 4 partitions: 1 / 2 / 4 / 8 waves 160 / 112 / 101 / 100 us).  Blocks along y do not
-    // count: longer ranges are longer chains, and the ranges of a row of 100 000 entries join within a warp.
-    int spg = slots_per_group();
+    // rows, 64 features, 4 partitions: 1 / 2 / 4 / 8 waves 160 / 112 / 101 / 100 us).  Blocks along y count for
+    // ranges, where their sums have two levels, and not for chains, which a row's error follows.
+    int spg = slots_per_group(), chain = 1 << 30;   // a range that was asked for is one chain
     if (!spg) {
       const int64_t want_tiles = (int64_t)sm_count() * min_blocks() * (f == Form::kGroups ? 4 : 8);
-      for (spg = 256; spg > 32; spg >>= 1) {
-        int64_t t = 0;
-        for (int k = 0; k < A->num_buckets; ++k) {
-          if (!in_pass(k)) continue;
-          const int w = A->widths[k];
-          const int rpg = spg / w > 0 ? spg / w : 1;
-          t += ceil_div64(A->ell_rows[k], (int64_t)rpg * gpc);
+      auto range = [&](int64_t along_y) {
+        int s = 256;
+        for (; s > 32; s >>= 1) {
+          int64_t t = 0;
+          for (int k = 0; k < A->num_buckets; ++k) {
+            if (!in_pass(k)) continue;
+            const int w = A->widths[k];
+            const int rpg = s / w > 0 ? s / w : 1;
+            t += ceil_div64(A->ell_rows[k], (int64_t)rpg * gpc);
+          }
+          if (t * along_y >= want_tiles) break;
         }
-        if (t >= want_tiles) break;
-      }
+        return s;
+      };
+      spg = chain = range(1);
+      if (f == Form::kGroups && group.G == 16 && group.passes > 1) spg = range(group.passes);
     }
     int i = 0;
     while (i < A->num_buckets) {
@@ -1204,11 +1214,12 @@ static int spmm_hyb_impl(const lf_hyb* A, const void* B, bool b_is_bf16, int64_t
         small.n = n;
         small.seg_tiles = (int32_t)(segs > 0 ? seg_tiles : 0);
         for (int k = 0; k < n; ++k) small.b[k] = big.b[k];
-        s = launch_hyb<16>(small, grid_tiles, A, B, ldb, C, ldc, N, cfg, f, group, st, dests, cleared_by_kernel);
+        s = launch_hyb<16>(small, grid_tiles, A, B, ldb, C, ldc, N, cfg, f, group, chain, st, dests, cleared_by_kernel);
       } else {
         big.n = n;
         big.seg_tiles = (int32_t)(segs > 0 ? seg_tiles : 0);
-        s = launch_hyb<LF_MAX_BUCKETS_PER_LAUNCH>(big, grid_tiles, A, B, ldb, C, ldc, N, cfg, f, group, st, dests, cleared_by_kernel);
+        s = launch_hyb<LF_MAX_BUCKETS_PER_LAUNCH>(big, grid_tiles, A, B, ldb, C, ldc, N, cfg, f, group, chain, st, dests,
+                                                  cleared_by_kernel);
       }
       if (s) return s;
       cleared_by_kernel = false;   // a further launch follows a product kernel, not the clearing one

@@ -71,6 +71,19 @@ def test_rows_of_one_ell_row(cuda_device, n, dtype, N, chains):
     assert _rms(got[:, :8], exact) <= 1.03 * _rms(_interleaved(vals, X, chains), exact)
 
 
+@pytest.mark.parametrize("N", [200, 512])
+def test_rows_of_eight_ell_rows_with_blocks_along_y(cuda_device, N):
+    """2^20 slots: chains are the ranges of 32 slots, although longer ranges fill the chip."""
+    csr, cols, vals = _matrix(4096, 256, cuda_device, 8)
+    fmt = hyb.build_hyb_device(csr, [[32]], with_mask=False)
+    B = _features(N, "float32", cuda_device)
+    X = B[:, :8][cols]
+    exact = (X.double() * vals.double()[:, :, None]).sum(1)
+    got = hyb.spmm_hyb(fmt, B)
+    assert hyb.spmm_hyb_kernel_name(fmt, B, got) == "spmm_hyb_groups_kernel"
+    assert _rms(got[:, :8], exact) <= 1.03 * _rms(_ranges(vals, X, 32), exact)
+
+
 @pytest.mark.parametrize("dtype,N,chains", [("float32", 32, 4), ("float32", 64, 2), ("bfloat16", 64, 4)])
 def test_long_rows(cuda_device, dtype, N, chains):
     """Rows shared by hundreds of ranges: the sums of 32 entries a range, added one behind the other."""
