@@ -637,18 +637,20 @@ spmm_hyb_ring_rows_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int
 // ---- a row of B per group of lanes ----------------------------------------------------------------
 // The form for a B that stays in the L2, where instructions per row bound the time: every group of
 // lanes, as narrow as a row of B, walks ELL rows of its own through the group ring (lf_spmm_group.cuh),
-// one launch for buckets of any width.  A row's error is no larger than in the forms for a larger B: those
-// keep four partial sums per row of up to 32 float32 (64 bf16) features, two up to 64 (128), one beyond.
+// one launch for buckets of any width.  A row's error is no larger than in the forms that take the product
+// without this one: from LF_OPT_SPMM_RING_MIN_SLOTS slots on those keep four partial sums per row of up to 32
+// float32 (64 bf16) features, two up to 64 (128), one beyond; smaller products add up one chain (ONE).
 // Batches cost registers: 32 features, at most 64 registers a thread / 80, three blocks per SM: 2^18
-// power-law rows 60 / 50 us, uniform rows 110 / 89 (one chain, error 1.3 to 2 times as large: 47, 85).
+// power-law rows 60 / 50 us, uniform rows 110 / 89 (one chain, error 1.3 to 2 times as large: 47, 85).  38 000 skewed
+// rows at 20 features, just above the threshold, 19.4 in one chain, 20.8.
 // Rows of more than 64 features have two levels: chains of `chain` slots, the ranges of the ring per warp, in
 // ranges that may be longer where there are blocks along y: 80 000 power-law rows at 256 features, one level
 // 86.5 us, two 79.7; 100 000 Zipf rows at 200 with 2 partitions 146, 135.
-template <int G, int CH> constexpr int kGroupSums = CH == 1 ? 3 : 2;
+template <int G, int CH, bool ONE> constexpr int kGroupSums = ONE ? 1 : (CH == 1 ? 3 : 2);
 template <int G> constexpr int kGroupBatch = G == 16 ? 0 : 4;
 
-template <int G, int CH, int VEC, int MAXB>
-__global__ void __launch_bounds__(kThreads, 3)
+template <int G, int CH, int VEC, bool ONE, int MAXB>
+__global__ void __launch_bounds__(kThreads, CH == 1 && ONE ? 4 : 3)
 spmm_hyb_groups_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int32_t* __restrict__ rows_arena,
                        const int32_t* __restrict__ cols_arena, const float* __restrict__ vals_arena,
                        const typename BTraits<VEC>::elem* __restrict__ B, int ldb, float* __restrict__ C, int64_t ldc,
@@ -667,7 +669,7 @@ spmm_hyb_groups_kernel(const __grid_constant__ SpmmTable<MAXB> tbl, const int32_
   ids.init(rows_arena + d.row_off, wlog, e0, e1, d.ell_rows);
   const int f0 = blockIdx.y * kFeatures;
 #define LF_WALK(WC_)                                                                                            \
-  walk_group_ring<G, CH, VEC, false, WC_, kGroupSums<G, CH>, kGroupBatch<G>>(                                                 \
+  walk_group_ring<G, CH, VEC, false, WC_, kGroupSums<G, CH, ONE>, kGroupBatch<G>>(                                                 \
       ids, d.force_atomic != 0, cols_arena + at, vals_arena + at, B + f0, ldb, C - row_base * ldc + f0, ldc,    \
       min(N - f0, kFeatures), g, gl, ring_bytes + w * GroupSmem<G, CH, false>::kBytes, max(chain, 1 << wlog))
   if (wlog == 0) LF_WALK(1);
@@ -868,19 +870,21 @@ template <int MAXB, int VEC>
 int launch_hyb_groups(const SpmmTable<MAXB>& tbl, int64_t tiles, const lf_hyb* A, const void* B, int64_t ldb, float* C,
                       int64_t ldc, int N, GroupCfg group, int chain, cudaStream_t st, bool dep) {
   const dim3 grid((unsigned)tiles, (unsigned)group.passes);
-#define LF_GROUPS(G_, CH_)                                                                                      \
+  const bool one = A->slot_off[A->num_buckets] < g_ring_rows_min_slots;
+#define LF_GROUPS(G_, CH_, ONE_)                                                                                    \
   do {                                                                                                          \
-    constexpr auto kern = spmm_hyb_groups_kernel<G_, CH_, VEC, MAXB>;                                           \
+    constexpr auto kern = spmm_hyb_groups_kernel<G_, CH_, VEC, ONE_, MAXB>;                                         \
     constexpr int smem = kThreads / 32 * GroupSmem<G_, CH_, false>::kBytes;                                     \
     LF_CUDA_CHECK(allow_smem<kern>(smem));                                                                      \
     LF_CUDA_CHECK(launch_dep_smem(kern, grid, kThreads, smem, st, dep, tbl, A->rows, A->cols, A->vals,          \
                                   (const typename BTraits<VEC>::elem*)B, (int)ldb, C, ldc, N, A->row_begin, chain)); \
     return LF_OK;                                                                                               \
   } while (0)
-  if (group.G == 4) LF_GROUPS(4, 1);
-  else if (group.G == 8 && group.CH == 1) LF_GROUPS(8, 1);
-  else if (group.G == 8) LF_GROUPS(8, 2);
-  else LF_GROUPS(16, 2);
+  if (group.G == 4) { if (one) LF_GROUPS(4, 1, true); else LF_GROUPS(4, 1, false); }
+  else if (group.G == 8 && group.CH == 1) { if (one) LF_GROUPS(8, 1, true); else LF_GROUPS(8, 1, false); }
+  else if (group.G == 8 && VEC == 8) LF_GROUPS(8, 2, true);   // bf16 rows of this width come in small products only
+  else if (group.G == 8) { if (one) LF_GROUPS(8, 2, true); else LF_GROUPS(8, 2, false); }
+  else LF_GROUPS(16, 2, false);
 #undef LF_GROUPS
 }
 

@@ -7,7 +7,7 @@ more than 100 000 sums is known to 0.2 %, so a product passes with up to 3 % mor
 import numpy as np
 import pytest
 
-from liteform_ae_b200 import hyb
+from liteform_ae_b200 import _cabi, hyb
 
 pytestmark = pytest.mark.gpu
 K = 20_000
@@ -60,15 +60,30 @@ def _features(N, dtype, device):
 @pytest.mark.parametrize("dtype,N,chains", [("float32", 16, 4), ("float32", 32, 4), ("float32", 64, 2), ("float32", 128, 1),
                                             ("bfloat16", 32, 4), ("bfloat16", 64, 4), ("bfloat16", 128, 2)])
 def test_rows_of_one_ell_row(cuda_device, n, dtype, N, chains):
-    csr, cols, vals = _matrix(16384 if n <= 64 else 4096, n, cuda_device, n)
+    """2^20 slots and more, from where the forms for a larger B keep several partial sums."""
+    csr, cols, vals = _matrix(max(4096, (1 << 20) // n), n, cuda_device, n)
     fmt = hyb.build_hyb_device(csr, [[n]], with_mask=False)
     B = _features(N, dtype, cuda_device)
     X = B[:, :8].float()[cols]
     exact = (X.double() * vals.double()[:, :, None]).sum(1)
     got = hyb.spmm_hyb(fmt, B)
-    if dtype == "float32" and N <= 64:
-        assert hyb.spmm_hyb_kernel_name(fmt, B, got) == "spmm_hyb_groups_kernel"
+    assert (hyb.spmm_hyb_kernel_name(fmt, B, got) == "spmm_hyb_groups_kernel") == (N <= 64)
     assert _rms(got[:, :8], exact) <= 1.03 * _rms(_interleaved(vals, X, chains), exact)
+
+
+@pytest.mark.parametrize("n", [5, 32, 64])
+@pytest.mark.parametrize("dtype,N", [("float32", n) for n in (12, 32, 64, 128, 260)] + [("bfloat16", n) for n in (32, 64, 128)])
+def test_small_products_have_the_sums_of_the_register_kernel(cuda_device, n, dtype, N):
+    csr, cols, vals = _matrix(2000, n, cuda_device, n)
+    fmt = hyb.build_hyb_device(csr, [[8, 32] if n < 64 else [64]], with_mask=False)
+    B = _features(N, dtype, cuda_device)
+    got, lib = hyb.spmm_hyb(fmt, B), _cabi.load()
+    assert hyb.spmm_hyb_kernel_name(fmt, B, got) == "spmm_hyb_groups_kernel"
+    assert lib.lf_set_option(_cabi.LF_OPT_SPMM_GATHER_RING, 0) == 0
+    try:
+        assert (got == hyb.spmm_hyb(fmt, B)).all()
+    finally:
+        lib.lf_set_option(_cabi.LF_OPT_SPMM_GATHER_RING, 16)
 
 
 @pytest.mark.parametrize("N", [200, 512])
