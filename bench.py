@@ -760,8 +760,8 @@ def roofline_of(prob, rec, world):
             "kernel": prob.kernel, "algorithmic_bytes_per_launch": int(alg), "launch_ms": launch_ms,
             "launch_ms_median": statistics.median(rec["step_ms_rank0"]),
             "gather_model_bytes_per_launch": int(gath), "gather_model_gbs": gath / (launch_ms * 1e-3) / 1e9,
-            # bytes every stored entry / block pulls out of L2 or HBM, per clock and SM at 148 SMs x 1965 MHz: the
-            # scattered-row gathers of these kernels top out near 30 (measured on the block workload)
+            # bytes every stored entry / block pulls out of L2 or HBM, per clock and SM at 148 SMs x 1965 MHz (30 in
+            # the float32 block kernel, 46 in the ring per warp on the power-law graph)
             "gather_model_bytes_per_clk_per_sm": gath / (launch_ms * 1e-3) / (148 * world * 1.965e9)}
 
 

@@ -85,11 +85,14 @@ const char* lf_last_error(void);
 #define LF_OPT_BSR_BLOCK_WARPS 11       /* copy engine 1, more than 64 features: warps per thread block, 1..8 (0 = automatic:
                                           4 for 16-bit inputs up to 128 features, else 8) */
 #define LF_OPT_SPMM_RING_MIN_SLOTS 12    /* stored slots from which a product whose B outgrows the L2 may take consecutive
-                                          slots per step, in two launches (default 2^20; 0: every product with
-                                          128-bit gathers does, whatever the size of B) */
+                                          slots per step, in two launches, and a row's sum is kept in several parts
+                                          (default 2^20; 0: every product with 128-bit gathers takes consecutive
+                                          slots, whatever the size of B) */
 #define LF_OPT_SPMM_GATHER_RING 10      /* products with 128-bit gathers: where the gathered rows of B land: 16 (default) a
-                                          ring of 16 rows (or steps of 2 / 4 narrow rows) per warp in shared memory,
-                                          filled by cp.async; 0 registers (8 rows in flight per warp) */
+                                          ring per warp in shared memory, filled by cp.async (16 rows, or steps of
+                                          2 / 4 narrow rows; 8 steps of a row per group of 4 to 16 lanes while B
+                                          stays in the L2; the CSR product: 8 steps of a row per group of 4 to 32
+                                          lanes); 0 registers (8 rows in flight per warp) */
 #define LF_OPT_SPMM_TILE_SEGMENTS 6     /* order of the thread blocks of the composed-format product: 0 bucket after
                                           bucket (default); S > 0: every bucket is cut into S segments of consecutive
                                           rows and the launch runs segment 0 of all buckets, then segment 1, ... */
@@ -294,6 +297,9 @@ int lf_spmm_hyb_f32_host(const lf_hyb* A_host /* rows/cols/vals/zero_rows are [h
  * format fails (proc05.spmm.end-to-end.py:237-249).  Work is split by stored entries, not by
  * rows: a long row is shared by many thread groups (vector atomics into rows that a preparation
  * launch cleared) and short rows are packed together, so no format has to be built first.
+ * Where N, ldb, ldc, B or C is off the 16-byte grid, rows of B are read in the aligned 16-byte pieces that
+ * cover them: up to 12 bytes before B and behind its last row are read (and not used), never beyond the
+ * 16-byte piece, hence never outside the pages of B.
  * ------------------------------------------------------------------------------------------- */
 int lf_spmm_csr_f32(const int64_t* indptr /*[dev]*/, const int32_t* indices /*[dev]*/,
                     const float* data /*[dev] or NULL: all ones*/, int64_t row_begin, int64_t row_end,
